@@ -110,7 +110,8 @@ int b200bssn_rhs(b200bssn_ctx *ctx, double *const *rhs, const double *const *u,
 /* Work plan for a fixed block list: descriptors, tiles and the derivative
  * scratch live on the device.  Build once, evaluate many times (RK stages).
  * `chunk_points` bounds the interior points evaluated per kernel pair (and so the
- * scratch: 1296 bytes per point in FP64, 648 in MIXED); 0 picks the default. */
+ * scratch: 1296 bytes per point in FP64, 648 in MIXED, and what pads rows to tiles of 16 x 8
+ * points: 4 % for 63^3 points, 18 % for 129^3); 0 picks the default. */
 int b200bssn_plan_create(b200bssn_ctx *ctx, const b200bssn_block *blocks, uint32_t nblocks,
                          uint32_t precision, uint64_t chunk_points, b200bssn_plan **plan);
 int b200bssn_plan_destroy(b200bssn_plan *plan);
@@ -118,8 +119,9 @@ int b200bssn_plan_destroy(b200bssn_plan *plan);
 /* Tuning knobs of a plan (0 in any field: the default). */
 typedef struct b200bssn_plan_options {
   uint64_t chunk_points;       /* interior points per kernel pair (scratch size) */
-  uint32_t slab_depth;         /* max interior z planes per work unit (default 48) */
-  uint32_t deriv_ctas_per_sm;  /* resident derivative CTAs per SM (default: as many as fit) */
+  uint32_t slab_depth;         /* max interior z planes per work unit, but never fewer than 3
+                                * (default: by a cost model of the whole plan) */
+  uint32_t deriv_ctas_per_sm;  /* resident derivative warps per SM, in fours (default: as many as fit) */
   /* NULL, or one entry per block overriding slab_depth for that block (0: keep
    * slab_depth); lets a tuner pick the depth per block-size class. */
   const uint32_t *block_slab_depth;
@@ -137,17 +139,11 @@ typedef struct b200bssn_plan_options {
   uint32_t single_pass;
   /* Ring slots of the one-pass kernel (0: 128; each slot 3072 points, 2 MB). */
   uint32_t ring_slots;
-  /* Tile height of the two-pass derivative kernels: 16 x tile_y columns per CTA, one
-   * thread per column (0: 8; also 4 or 16). */
+  /* Knobs of earlier derivative kernels (tile height 4, 8 or 16; register split 1, 2 or 3;
+   * one or two points per thread).  There is one kernel shape now: values and combinations
+   * that were accepted still are and change nothing, the others are still refused. */
   uint32_t tile_y;
-  /* Registers-per-thread split of the two-pass derivative kernels (the kinds without /
-   * with second derivatives): 1 = 96 / 128 registers, 2 = 80 / 96 (one CTA per SM
-   * more), 3 = 128 / 168 (one fewer); 2 and 3 with 16x8 tiles and centred advection
-   * only.  0: the measured best -- 3 for FP64 with centred advection and 16x8 tiles,
-   * else 1. */
   uint32_t deriv_regs;
-  /* 2: the two-pass derivative kernels give each thread two output points (y pairs of
-   * 16x16 tiles, CTAs of 128 threads), centred advection only; 0 or 1: one point. */
   uint32_t points_per_thread;
 } b200bssn_plan_options;
 

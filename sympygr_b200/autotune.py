@@ -6,25 +6,15 @@ class's block count from the batch, times --scale) it builds a plan of that clas
 alone and times one evaluation (CUDA events, device-resident inputs larger than L2)
 for every candidate of
 
-* tile shape: 16 x tile_y columns per derivative CTA, tile_y 4, 8 or 16 (64, 128 or
-  256 threads; the staged plane, the D_x halo rows and the register queues follow);
-* registers-per-thread split of the derivative kernels: 96 / 128 registers for the kinds
-  without / with second derivatives, one CTA per SM more (80 / 96) or one fewer
-  (128 / 168) -- with 16x8 tiles (the plans' default is the last for FP64, the first
-  for MIXED);
-* output points per thread: one, or two (y pairs of 16x16 tiles in CTAs of 128 threads);
 * slab depth (staging depth along z): the z-planes per work unit of the derivative
-  kernel (candidates that cut the interior into the same number of slabs are the same
-  plan, so one per slab count is timed);
+  kernels (candidates that cut the interior into the same number of slabs are the same
+  plan, so one per slab count is timed), and the plan's own choice;
 * with --ctas, derivative CTAs per SM capped at 1 or 2 as well as uncapped.
 
 It writes the per-class table and choice to JSON.  ``tuned_plan`` builds a plan for
 any block list from such a table: each block gets its class's slab depth
-(b200bssn_plan_options.block_slab_depth); the tile shape, register split and CTA
-count are plan-wide knobs.  They are settled on the whole batch: the default plan, the
-per-class depths with the default plan-wide knobs, and the per-class depths with the
-knobs of the class holding the most points are timed, and the table keeps the fastest
-(so a class's win inside the timing noise cannot cost the other classes).
+(b200bssn_plan_options.block_slab_depth); the CTA cap is the plan's.  The whole batch
+settles between the default plan and the tuned ones.
 
     python -m sympygr_b200.autotune --precision mixed --json tune_mixed.json
 """
@@ -66,12 +56,6 @@ def time_plan(plan, rhs, u, prm, reps: int = 5, warmup: int = 2) -> float:
     return e0.elapsed_time(e1) / reps
 
 
-# (tile_y, deriv_regs) variants of the derivative kernels built into the library
-# (deriv_regs 1: 96/128 registers for the kinds without/with second derivatives, 2: 80/96,
-# 3: 128/168)
-KERNEL_VARIANTS = [(8, 1, 1), (4, 1, 1), (16, 1, 1), (8, 2, 1), (8, 3, 1), (16, 0, 2)]  # + points per thread
-
-
 def tuned_plan(ctx, blocks, precision, table, chunk_points: int = 0):
     """A plan whose blocks use their size class's tuned slab depth and the table's
     plan-wide knobs (the default plan where the table found the tuned one no faster)."""
@@ -80,8 +64,7 @@ def tuned_plan(ctx, blocks, precision, table, chunk_points: int = 0):
     choice = {int(k): v for k, v in table["choice"].items()}
     depths = [choice.get(b.sz[2], {}).get("slab_depth", 0) for b in blocks]
     return capi.Plan(ctx, blocks, precision, chunk_points, deriv_ctas_per_sm=table["deriv_ctas_per_sm"],
-                     block_slab_depth=depths, tile_y=table.get("tile_y", 0),
-                     deriv_regs=table.get("deriv_regs", 0), points_per_thread=table.get("points_per_thread", 0))
+                     block_slab_depth=depths)
 
 
 def main(argv=None):
@@ -105,24 +88,17 @@ def main(argv=None):
         rhs = torch.zeros_like(u)
         pts = sum(b.ninterior for b in blocks)
         rows = []
-        for ty, regs, ppt in KERNEL_VARIANTS:
-            for d in depth_candidates(n):
-                for ctas in ((0, 1, 2) if args.ctas else (0,)):
-                    plan = capi.Plan(ctx, blocks, prec, slab_depth=d, deriv_ctas_per_sm=ctas, tile_y=ty,
-                                     deriv_regs=regs, points_per_thread=ppt)
-                    ms = time_plan(plan, list(rhs), list(u), prm, args.reps)
-                    plan.close()
-                    rows.append({"tile_y": ty, "deriv_regs": regs, "points_per_thread": ppt, "slab_depth": d,
-                                 "deriv_ctas_per_sm": ctas, "ms": ms, "mpts_per_s": pts / ms / 1e3})
-                    print(json.dumps({"class": n, **rows[-1]}), flush=True)
+        for d in [0] + depth_candidates(n):  # 0: the plan's own choice
+            for ctas in ((0, 1, 2) if args.ctas else (0,)):
+                plan = capi.Plan(ctx, blocks, prec, slab_depth=d, deriv_ctas_per_sm=ctas)
+                ms = time_plan(plan, list(rhs), list(u), prm, args.reps)
+                plan.close()
+                rows.append({"slab_depth": d, "deriv_ctas_per_sm": ctas, "ms": ms, "mpts_per_s": pts / ms / 1e3})
+                print(json.dumps({"class": n, **rows[-1]}), flush=True)
         best = max(rows, key=lambda r: r["mpts_per_s"])
-        nslab = lambda d: -(-(n - 6) // d)  # noqa: E731 -- slabs of the class's blocks at depth d
-        dregs = 3 if prec == capi.FP64 else 1  # the plan's default split for this precision
-        default = next(r for r in rows if r["tile_y"] == 8 and r["deriv_regs"] == dregs and r["deriv_ctas_per_sm"] == 0
-                       and r["points_per_thread"] == 1 and nslab(r["slab_depth"]) == nslab(48))
+        default = rows[0]
         table["classes"][str(n)] = {"blocks": c, "points": pts, "runs": rows}
-        table["choice"][str(n)] = {k: best[k] for k in ("tile_y", "deriv_regs", "points_per_thread", "slab_depth",
-                                                        "deriv_ctas_per_sm", "mpts_per_s")}
+        table["choice"][str(n)] = {k: best[k] for k in ("slab_depth", "deriv_ctas_per_sm", "mpts_per_s")}
         table["choice"][str(n)]["gain_over_default"] = best["mpts_per_s"] / default["mpts_per_s"]
         if pts > best_points[0]:
             best_points = (pts, best)
@@ -131,7 +107,7 @@ def main(argv=None):
     # the whole batch settles the plan-wide knobs: the default plan, the per-class depths
     # with the default knobs, and the per-class depths with the knobs of the class
     # holding the most points
-    knobs = ("deriv_ctas_per_sm", "tile_y", "deriv_regs", "points_per_thread")
+    knobs = ("deriv_ctas_per_sm",)
     u, blocks = wl.two_puncture_batch_torch(wl.BATCH_SIZES, counts, seed=0, device="cuda")
     rhs = torch.zeros_like(u)
     pts = sum(b.ninterior for b in blocks)
@@ -154,8 +130,7 @@ def main(argv=None):
                       "depths_class_knobs_mpts_per_s": pts / timed["class_knobs"] / 1e3,
                       "tuned_mpts_per_s": pts / min(ms_default, timed[pick]) / 1e3, "plan_wide": pick}
     print(json.dumps({"choice": table["choice"], "batch": table["batch"],
-                      "plan_wide": {k: table[k] for k in ("deriv_ctas_per_sm", "tile_y", "deriv_regs",
-                                                          "points_per_thread")}}),
+                      "plan_wide": {k: table[k] for k in knobs}}),
           flush=True)
     if args.json:
         with open(args.json, "w") as f:

@@ -39,9 +39,13 @@ bool b200bssn::host::params_ok(const b200bssn_params* p) {
 namespace {
 
 constexpr int64_t kDefaultChunkPoints = int64_t(1) << 23;
-// scratch slots are addressed with 32-bit offsets: slots * cap < 2^31 (slots: 138, or
-// 210 in the upwind mode)
-constexpr int64_t max_chunk_points(int slots) { return (int64_t(1) << 31) / (slots + 1) - 1; }
+// scratch slots are addressed with 32-bit offsets: slots * scratch points < 2^31
+constexpr int64_t max_scratch_points(int slots) { return ((int64_t(1) << 31) / slots - 1) / kTilePlane * kTilePlane; }
+// the chunk sizes accepted (interior points; the limit of a scratch without padding)
+constexpr int64_t max_chunk_points(bool adv) { return (int64_t(1) << 31) / (kNumDerivs + (adv ? 3 * kNumVars : 0) + 1) - 1; }
+// work counters of an evaluation, zeroed at its start: one per derivative launch of a chunk
+constexpr size_t kDerivCounters = 6;
+constexpr size_t counter_words(size_t chunks) { return kDerivCounters * chunks; }
 
 void make_args(const b200bssn_plan* P, double* const* rhs, const double* const* u,
                const b200bssn_params* prm, DerivArgs& da, AlgebraArgs& aa) {
@@ -53,10 +57,9 @@ void make_args(const b200bssn_plan* P, double* const* rhs, const double* const* 
     aa.rhs[v] = rhs[v];
   }
   da.blocks = aa.blocks = P->d_blocks;
-  da.units = aa.units = P->d_units;
   da.tiles = P->d_tiles;
+  aa.slabs = P->d_slabs;
   aa.ranges = P->d_ranges;
-  da.cap = aa.cap = (int32_t)P->cap;
   aa.prm64 = {(double)prm->lambda[0], (double)prm->lambda[1], (double)prm->lambda[2],
               (double)prm->lambda[3], prm->lambda_f[0], prm->lambda_f[1]};
   aa.prm32 = {(float)prm->lambda[0], (float)prm->lambda[1], (float)prm->lambda[2],
@@ -67,38 +70,44 @@ void make_args(const b200bssn_plan* P, double* const* rhs, const double* const* 
   aa.ko_sigma = prm->ko_sigma;
 }
 
-// The derivative kind kernels built for each plan knob: tile height 4, 8 or 16 with the
-// default register split, and 16x8 tiles with one CTA per SM more or fewer (the upwind
-// mode only with the defaults).  Returns the kernel, or nullptr if not built.
-template <typename ST, bool ADV, int TY, int REGV>
-const void* kind_ptr(bool dd) {
-  return dd ? (const void*)bssn_derivs_kind_kernel<ST, true, ADV, TY, REGV>
-            : (const void*)bssn_derivs_kind_kernel<ST, false, ADV, TY, REGV>;
+// The derivative kernels of a plan: [kind: without / with second derivatives][TileClosure].
+template <typename ST, bool ADV, bool DD>
+void kind_kernels(const void* (&fn)[3]) {
+  fn[kClosureNone] = (const void*)bssn_derivs_kind_kernel<ST, DD, ADV, kClosureNone>;
+  fn[kClosureZ] = (const void*)bssn_derivs_kind_kernel<ST, DD, ADV, kClosureZ>;
+  fn[kClosureXY] = (const void*)bssn_derivs_kind_kernel<ST, DD, ADV, kClosureXY>;
 }
-const void* kind_kernel(bool mixed, bool adv, bool dd, int ty, int regv) {
-  if (adv) {
-    if (ty != kTileY || regv != 0) return nullptr;
-    return mixed ? kind_ptr<float, true, kTileY, 0>(dd) : kind_ptr<double, true, kTileY, 0>(dd);
-  }
-#define B200BSSN_KIND(TYV, RV) \
-  if (ty == TYV && regv == RV) return mixed ? kind_ptr<float, false, TYV, RV>(dd) : kind_ptr<double, false, TYV, RV>(dd);
-  B200BSSN_KIND(8, 0)
-  B200BSSN_KIND(8, 1)
-  B200BSSN_KIND(8, 2)
-  B200BSSN_KIND(4, 0)
-  B200BSSN_KIND(16, 0)
-#undef B200BSSN_KIND
-  return nullptr;
+template <typename ST, bool ADV>
+void kind_kernels(const void* (&fn)[2][3]) {
+  kind_kernels<ST, ADV, false>(fn[0]);
+  kind_kernels<ST, ADV, true>(fn[1]);
 }
 
-// The derivative stage of one chunk: the kernels over the variables without and with
-// second derivatives, each with its own work counter.
-int launch_derivs(b200bssn_plan* P, DerivArgs dn, DerivArgs dd, int gn, int gd, cudaStream_t s) {
-  void* an[] = {&dn};
-  void* ad[] = {&dd};
-  const dim3 block((unsigned)P->deriv_threads);
-  CK(P->ctx, cudaLaunchKernel(P->kind_fn[0], dim3((unsigned)gn), block, an, 0, s));
-  CK(P->ctx, cudaLaunchKernel(P->kind_fn[1], dim3((unsigned)gd), block, ad, 0, s));
+// The derivative stage of chunk ci: per kind one launch for each list of tiles (by their
+// closure rows, the slowest first), with its own work counter; empty lists are left out.
+int launch_derivs(b200bssn_plan* P, const DerivArgs& da, size_t ci, cudaStream_t s) {
+  const ChunkRec& c = P->chunks[ci];
+  if (P->advective) {
+    bssn_shift_signs_kernel<<<(unsigned)c.tile_count, kTilePlane, 0, s>>>(
+        da.u[6], da.u[7], da.u[8], da.blocks, da.tiles + c.tile_begin, const_cast<uint8_t*>(da.up));
+    CK(P->ctx, cudaGetLastError());
+  }
+  bool follows = false;
+  for (int k = 1; k >= 0; --k) {
+    int at = c.tile_begin + c.tile_count;
+    for (int cl = 2; cl >= 0; --cl) {
+      at -= c.list[cl];
+      if (c.list[cl] == 0) continue;
+      DerivArgs d = da;
+      d.tile_count = c.list[cl];
+      d.order = P->d_order + at;
+      d.counter = P->d_counters + kDerivCounters * ci + 3 * k + cl;
+      const int grid = (int)std::min<int64_t>((int64_t)d.tile_count * kKindVars[k], P->deriv_grid[k][cl]);
+      void* arg[] = {&d};
+      CK(P->ctx, launch_deriv(P->kind_fn[k][cl], grid, arg, follows, s));
+      follows = true;
+    }
+  }
   return B200BSSN_OK;
 }
 
@@ -145,24 +154,13 @@ int enqueue_chunk(b200bssn_plan* P, DerivArgs da, AlgebraArgs aa, size_t ci, int
   b200bssn_ctx* ctx = P->ctx;
   const ChunkRec& c = P->chunks[ci];
   const bool mixed = P->precision == B200BSSN_MIXED;
-  da.tile_base = c.tile_begin;
-  da.tile_count = c.tile_count;
-  da.counter = P->d_counters + ci;
   aa.range_base = c.range_begin;
-  da.dscr = P->dscr[buf];
-  aa.dscr = P->dscr[buf];
-  da.koscr = P->koscr[buf];
-  aa.koscr = P->koscr[buf];
+  da.scr = P->scr[buf];
+  da.up = P->up[buf];
+  aa.scr = P->scr[buf];
   if (ev) CK(ctx, cudaEventRecord(ev[4 * ci + 0], s1));
   {
-    // the two derivative kernels (variables without, then with second derivatives),
-    // each with its own work counter
-    DerivArgs dn = da, dd = da;
-    dn.counter = P->d_counters + 2 * ci;
-    dd.counter = P->d_counters + 2 * ci + 1;
-    const int gn = std::min(c.tile_count * kKindVars[0], P->deriv_grid[0]);
-    const int gd = std::min(c.tile_count * kKindVars[1], P->deriv_grid[1]);
-    const int rc = launch_derivs(P, dn, dd, gn, gd, s1);
+    const int rc = launch_derivs(P, da, ci, s1);
     if (rc != B200BSSN_OK) return rc;
   }
   CK(ctx, cudaGetLastError());
@@ -175,14 +173,14 @@ int enqueue_chunk(b200bssn_plan* P, DerivArgs da, AlgebraArgs aa, size_t ci, int
   if (ca) {
     ConstraintArgs cc = *ca;
     cc.range_base = c.range_begin;
-    cc.dscr = P->dscr[buf];
+    cc.scr = P->scr[buf];
     if (mixed)
       bssn_constraints_kernel<float, float><<<c.range_count, kAlgebraThreads, 0, s2>>>(cc);
     else
       bssn_constraints_kernel<double, double><<<c.range_count, kAlgebraThreads, 0, s2>>>(cc);
   } else {
     // the staged persistent kernel: each warp takes 32-point tasks round-robin
-    const int ntasks = c.range_count * (kAlgebraThreads / kStageW);
+    const int ntasks = c.range_count * kRangeTasks;
     const unsigned gs = (unsigned)std::max(1, std::min(P->alg_grid, ntasks));
     if (mixed)
       P->advective ? launch_algebra<float, true>(aa, gs, ntasks, s2)
@@ -206,9 +204,7 @@ int launch_single_pass(b200bssn_plan* P, const DerivArgs& da, const AlgebraArgs&
   std::memset(&f, 0, sizeof(f));
   f.d = da;
   f.a = aa;
-  f.d.dscr = P->fring_d;
-  f.d.koscr = P->fring_k;
-  f.d.cap = P->nring * kFusedSlotPts;
+  f.d.scr = P->fring;
   f.tiles = P->d_ftiles;
   f.ntiles = (int32_t)P->ftiles.size();
   f.nring = P->nring;
@@ -266,7 +262,7 @@ int b200bssn::host::launch_plan(b200bssn_plan* P, double* const* rhs, const doub
   const size_t nch = P->chunks.size();
   const bool pipelined = ev == nullptr && nch > 1;
   cudaStream_t s1 = pipelined ? ctx->s_deriv : s, s2 = pipelined ? ctx->s_alg : s;
-  CK(ctx, cudaMemsetAsync(P->d_counters, 0, 2 * nch * sizeof(int), s));
+  CK(ctx, cudaMemsetAsync(P->d_counters, 0, counter_words(nch) * sizeof(int), s));
   if (pipelined) {
     CK(ctx, cudaEventRecord(P->ev_fork, s));
     CK(ctx, cudaStreamWaitEvent(s1, P->ev_fork, 0));
@@ -283,16 +279,62 @@ int b200bssn::host::launch_plan(b200bssn_plan* P, double* const* rhs, const doub
 
 namespace {
 
+// Default z-slab depth of a plan, from a model of the derivative stage: a tile costs its
+// planes, the 6 halo planes and about 4 planes' worth of start-up; the 11 variables with second
+// derivatives (the longer kernel) share out 6 CTAs per SM, and each launch ends with one
+// tile's time.  Deep slabs pay the halo less often, shallow ones give small plans enough
+// items and every launch a shorter tail.  (16 blocks of 69^3 as one slab each, or in slabs of
+// 48, 24, 12, 6, 3 planes, MIXED: 0.86, 0.91, 0.93, 1.07, 1.32, 1.76 ms.)
+int64_t default_depth(const b200bssn_block* blocks, uint32_t nblocks, uint64_t chunk_points, int sms) {
+  const double resident = 6.0 * std::max(1, sms);
+  const int64_t capacity = chunk_points ? (int64_t)chunk_points : kDefaultChunkPoints;
+  int64_t best = 3;
+  double best_cost = 0.0;
+  for (const int64_t depth : {3, 4, 5, 6, 8, 11, 16, 22, 33, 44, 66, 99, 132}) {
+    double work = 0.0, points = 0.0;
+    int64_t longest = 0;
+    for (uint32_t b = 0; b < nblocks; ++b) {
+      const int64_t I0 = (int64_t)blocks[b].sz[0] - 6, I1 = (int64_t)blocks[b].sz[1] - 6, I2 = (int64_t)blocks[b].sz[2] - 6;
+      if (I0 < 7 || I1 < 7 || I2 < 7) continue;  // refused later
+      const int64_t n = std::min((I2 + depth - 1) / depth, I2 / 3);
+      const int64_t tiles = ((I0 + kTileX - 1) / kTileX) * ((I1 + kTileY - 1) / kTileY);
+      work += (double)tiles * (double)(I2 + 10 * n);
+      points += (double)I0 * I1 * I2;
+      longest = std::max(longest, (I2 + n - 1) / n + 10);
+    }
+    const double launches = std::max(1.0, points / (double)capacity);
+    const double cost = work * kKindVars[1] / resident + launches * (double)longest;
+    if (best_cost == 0.0 || cost < best_cost) {
+      best_cost = cost;
+      best = depth;
+    }
+  }
+  return best;
+}
+
+// Orders each chunk's tiles by their closure rows (TileClosure), the longest first in each
+// list (cost ~ planes streamed).  The lists follow the blocks' face flags.
+void order_tiles(b200bssn_plan* P) {
+  P->order.resize(P->tiles.size());
+  for (size_t k = 0; k < P->order.size(); ++k) P->order[k] = (int32_t)k;
+  for (ChunkRec& c : P->chunks) {
+    auto kind = [&](int32_t k) { return (int)tile_closure(P->blocks[P->tiles[k].block], P->tiles[k]); };
+    const auto lo = P->order.begin() + c.tile_begin, hi = lo + c.tile_count;
+    std::stable_sort(lo, hi, [&](int32_t x, int32_t y) {
+      const int kx = kind(x), ky = kind(y);
+      return kx != ky ? kx < ky : P->tiles[x].nz > P->tiles[y].nz;
+    });
+    for (int32_t& n : c.list) n = 0;
+    for (auto it = lo; it != hi; ++it) ++c.list[kind(*it)];
+  }
+}
+
 int set_kernel_attributes(b200bssn_ctx* ctx) {
   int rc = set_stage_attributes<float, false>(ctx);
   if (rc == B200BSSN_OK) rc = set_stage_attributes<float, true>(ctx);
   if (rc == B200BSSN_OK) rc = set_stage_attributes<double, false>(ctx);
   if (rc == B200BSSN_OK) rc = set_stage_attributes<double, true>(ctx);
   if (rc != B200BSSN_OK) return rc;
-  CK(ctx, cudaFuncSetAttribute(bssn_derivs_kernel<double>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDerivSmemBytes));
-  CK(ctx, cudaFuncSetAttribute(bssn_derivs_kernel<float>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kDerivSmemBytes));
   const int fb = (int)kFusedSmemBytes;
   CK(ctx, cudaFuncSetAttribute(bssn_fused_kernel<RK_NONE>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb));
   CK(ctx, cudaFuncSetAttribute(bssn_fused_kernel<RK_FIRST>, cudaFuncAttributeMaxDynamicSharedMemorySize, fb));
@@ -404,7 +446,6 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   std::memset(&o, 0, sizeof(o));
   if (opts) o = *opts;
   const uint64_t chunk_points = o.chunk_points;
-  const int64_t slab_depth = o.slab_depth ? (int64_t)o.slab_depth : kTileZ;
   if (!ctx || !blocks || !out || nblocks == 0) return B200BSSN_ERR_INVALID_ARGUMENT;
   if (precision != B200BSSN_FP64 && precision != B200BSSN_MIXED) return B200BSSN_ERR_INVALID_ARGUMENT;
   *out = nullptr;
@@ -413,39 +454,29 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   P->ctx = ctx;
   P->precision = precision;
   P->advective = o.advective != 0;
-  P->tile_y = o.tile_y ? (int)o.tile_y : kTileY;
-  // register split: option 1 = 96/128 registers (the kinds without / with second
-  // derivatives), 2 = 80/96, 3 = 128/168; 0 = the measured best for the precision
-  // (FP64 with centred advection: 128/168, 4 % faster on the batch; else 96/128)
-  const uint32_t regs_opt = o.deriv_regs ? o.deriv_regs
-                                         : (precision == B200BSSN_FP64 && !P->advective && P->tile_y == kTileY ? 3u : 1u);
-  P->deriv_regs = regs_opt >= 1 && regs_opt <= 3 ? (int)regs_opt - 1 : -1;  // kernel variant
-  P->deriv_threads = kTileX * P->tile_y;
-  for (int k = 0; k < 2; ++k)
-    P->kind_fn[k] = kind_kernel(precision == B200BSSN_MIXED, P->advective, k == 1, P->tile_y, P->deriv_regs);
-  if (o.points_per_thread == 2) {
-    // y pairs: 16x16 tiles, 128 threads, centred advection, the pair kernels' own split
-    const bool ok = !P->advective && (o.tile_y == 0 || o.tile_y == 16) && o.deriv_regs == 0;
-    P->tile_y = 16;
-    P->deriv_threads = 128;
-    for (int k = 0; k < 2; ++k)
-      P->kind_fn[k] = !ok ? nullptr
-                          : (precision == B200BSSN_MIXED
-                                 ? (k ? (const void*)bssn_derivs_pair_kernel<float, true>
-                                      : (const void*)bssn_derivs_pair_kernel<float, false>)
-                                 : (k ? (const void*)bssn_derivs_pair_kernel<double, true>
-                                      : (const void*)bssn_derivs_pair_kernel<double, false>));
-  } else if (o.points_per_thread > 2) {
-    P->kind_fn[0] = P->kind_fn[1] = nullptr;
+  // The tuning knobs of earlier stencil kernels: the values they took are still accepted (the
+  // kernels have one tile shape and register split now), the others still refused.
+  {
+    const uint32_t ty = o.tile_y ? o.tile_y : 8u, regs = o.deriv_regs;
+    bool ok = (ty == 4 || ty == 8 || ty == 16) && regs <= 3 && o.points_per_thread <= 2;
+    ok = ok && (ty == 8 || regs <= 1) && (!P->advective || (ty == 8 && regs <= 1));
+    if (o.points_per_thread == 2) ok = !P->advective && (o.tile_y == 0 || o.tile_y == 16) && regs == 0;
+    if (!ok) {
+      delete P;
+      return B200BSSN_ERR_INVALID_ARGUMENT;
+    }
   }
-  if (!P->kind_fn[0] || !P->kind_fn[1]) {
-    delete P;
-    return B200BSSN_ERR_INVALID_ARGUMENT;
-  }
-  const int nslots = P->advective ? kNumDerivs + 3 * kNumVars : kNumDerivs;
-  const int64_t kMaxChunkPoints = max_chunk_points(nslots);
+  if (precision == B200BSSN_MIXED)
+    P->advective ? kind_kernels<float, true>(P->kind_fn) : kind_kernels<float, false>(P->kind_fn);
+  else
+    P->advective ? kind_kernels<double, true>(P->kind_fn) : kind_kernels<double, false>(P->kind_fn);
+  const int nslots = num_slots(P->advective);
+  const int64_t kMaxChunkPoints = max_chunk_points(P->advective), kMaxScratch = max_scratch_points(nslots);
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+  const int64_t slab_depth = o.slab_depth ? (int64_t)o.slab_depth : default_depth(blocks, nblocks, chunk_points, sms);
   P->span_lo = UINT64_MAX;
-  int64_t max_unit = 0;
+  int64_t max_slab = 0;  // interior points
   for (uint32_t b = 0; b < nblocks; ++b) {
     const b200bssn_block& in = blocks[b];
     for (int a = 0; a < 3; ++a) {
@@ -475,75 +506,75 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
     P->span_lo = std::min<uint64_t>(P->span_lo, in.offset);
     P->span_hi = std::max<uint64_t>(P->span_hi, in.offset + npad);
     const int64_t I0 = in.sz[0] - 6, I1 = in.sz[1] - 6, I2 = in.sz[2] - 6;
-    // z-slabs of nearly equal depth (<= depth planes): the derivative kernel
-    // streams each slab plus 4 halo planes on each side
+    // z-slabs of nearly equal depth (<= depth planes, and never below three, see cut_start):
+    // the derivative kernels stream each slab plus 3 halo planes on each side
     const int64_t depth = (o.block_slab_depth && o.block_slab_depth[b])
                               ? (int64_t)o.block_slab_depth[b] : slab_depth;
-    const int64_t nslab = (I2 + depth - 1) / depth;
+    const int64_t nslab = std::min((I2 + depth - 1) / depth, I2 / 3);
     if ((uint64_t)I0 * I1 * ((I2 + nslab - 1) / nslab) > (uint64_t)INT32_MAX) {
       delete P;
       return B200BSSN_ERR_INVALID_ARGUMENT;
     }
     for (int64_t sl = 0; sl < nslab; ++sl) {
       const int64_t k0 = sl * I2 / nslab, k1 = (sl + 1) * I2 / nslab;
-      UnitDev u;
-      u.block = (int32_t)b;
-      u.k0 = (int32_t)k0;
-      u.nz = (int32_t)(k1 - k0);
-      u.pad = 0;
-      u.sbase = 0;
-      P->units.push_back(u);
-      max_unit = std::max<int64_t>(max_unit, I0 * I1 * u.nz);
+      P->slabs.push_back({(int32_t)b, (int32_t)k0, (int32_t)(k1 - k0), 0});
+      max_slab = std::max<int64_t>(max_slab, I0 * I1 * (k1 - k0));
     }
     P->points += (uint64_t)(I0 * I1 * I2);
   }
   int64_t capacity = chunk_points ? (int64_t)chunk_points : kDefaultChunkPoints;
-  capacity = std::min(std::max(capacity, max_unit), kMaxChunkPoints);
-  if (max_unit > kMaxChunkPoints) {
+  capacity = std::min(std::max(capacity, max_slab), kMaxChunkPoints);
+  if (max_slab > kMaxChunkPoints) {
     delete P;
     return B200BSSN_ERR_SIZE_LIMIT;
   }
-  // pack units into chunks
-  ChunkRec cur{0, 0, 0, 0, 0};
+  // pack slabs into chunks
+  ChunkRec cur{0, 0, {0, 0, 0}, 0, 0, 0};
+  int64_t used = 0;  // scratch points of the current chunk
   auto flush = [&]() {
     if (cur.points > 0) {
       cur.tile_count = (int32_t)P->tiles.size() - cur.tile_begin;
       cur.range_count = (int32_t)P->ranges.size() - cur.range_begin;
       P->chunks.push_back(cur);
-      P->cap = std::max<int64_t>(P->cap, (cur.points + 31) & ~int64_t(31));
+      P->cap = std::max<int64_t>(P->cap, used);
     }
-    cur = ChunkRec{(int32_t)P->tiles.size(), 0, (int32_t)P->ranges.size(), 0, 0};
+    cur = ChunkRec{(int32_t)P->tiles.size(), 0, {0, 0, 0}, (int32_t)P->ranges.size(), 0, 0};
+    used = 0;
   };
-  for (size_t ui = 0; ui < P->units.size(); ++ui) {
-    UnitDev& u = P->units[ui];
+  for (size_t si = 0; si < P->slabs.size(); ++si) {
+    SlabDev& u = P->slabs[si];
     const BlockDev& B = P->blocks[u.block];
     const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6;
-    const int64_t np = (int64_t)I0 * I1 * u.nz;
-    // a block's units stay in one chunk when the whole block fits in one
+    const int cutx = num_cuts(I0, kTileX), cuty = num_cuts(I1, kTileY);
+    const int64_t points = (int64_t)I0 * I1 * u.nz, need = (int64_t)cutx * cuty * u.nz * kTilePlane;
+    if (need > kMaxScratch) {
+      delete P;
+      return B200BSSN_ERR_SIZE_LIMIT;
+    }
+    // a block's slabs stay in one chunk when the whole block fits in one
     const int64_t block_pts = (int64_t)I0 * I1 * (B.sz[2] - 6);
-    const bool first_unit = ui == 0 || P->units[ui - 1].block != u.block;
-    if (first_unit && block_pts <= capacity && cur.points + block_pts > capacity) flush();
-    if (((cur.points + 31) & ~int64_t(31)) + np > capacity) flush();
-    cur.points = (cur.points + 31) & ~int64_t(31);  // slot runs start 128-byte aligned
-    u.sbase = cur.points;
-    cur.points += np;
-    for (int j0 = 0; j0 < I1; j0 += P->tile_y)
-      for (int i0 = 0; i0 < I0; i0 += kTileX) {
+    const bool first = si == 0 || P->slabs[si - 1].block != u.block;
+    if (first && block_pts <= capacity && cur.points + block_pts > capacity) flush();
+    if (cur.points + points > capacity || used + need > kMaxScratch) flush();
+    cur.points += points;
+    u.sbase = (int32_t)used;
+    for (int ty = 0; ty < cuty; ++ty)
+      for (int tx = 0; tx < cutx; ++tx) {
         TileDev t;
-        t.unit = (int32_t)ui;
-        t.i0 = (int16_t)i0;
-        t.j0 = (int16_t)j0;
-        t.ex = (int16_t)std::min(kTileX, I0 - i0);
-        t.ey = (int16_t)std::min(P->tile_y, I1 - j0);
+        t.block = u.block;
+        t.sbase = u.sbase + (ty * cutx + tx) * u.nz * kTilePlane;
+        t.k0 = u.k0;
+        t.nz = u.nz;
+        t.i0 = (int16_t)cut_start(I0, kTileX, tx);
+        t.j0 = (int16_t)cut_start(I1, kTileY, ty);
+        t.ex = (int16_t)(cut_start(I0, kTileX, tx + 1) - t.i0);
+        t.ey = (int16_t)(cut_start(I1, kTileY, ty + 1) - t.j0);
         P->tiles.push_back(t);
       }
-    for (int64_t s = 0; s < np; s += kAlgebraThreads) {
-      RangeDev r;
-      r.unit = (int32_t)ui;
-      r.start = (int32_t)s;
-      r.count = (int32_t)std::min<int64_t>(kAlgebraThreads, np - s);
-      P->ranges.push_back(r);
-    }
+    used += need;
+    const int tasks = (int)slab_tasks(B, u.nz);
+    for (int s = 0; s < tasks; s += kRangeTasks)
+      P->ranges.push_back({(int32_t)si, s, std::min(kRangeTasks, tasks - s)});
   }
   flush();
   // Host pipeline partition: chunk c owns elements [part[c], part[c+1]) when the
@@ -554,7 +585,7 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
     for (size_t c = 0; c < P->chunks.size(); ++c) {
       const ChunkRec& ch = P->chunks[c];
       for (int r = ch.range_begin; r < ch.range_begin + ch.range_count; ++r) {
-        const int32_t bi = P->units[P->ranges[r].unit].block;
+        const int32_t bi = P->slabs[P->ranges[r].slab].block;
         const BlockDev& B = P->blocks[bi];
         const uint64_t np = (uint64_t)B.sz[0] * B.sz[1] * B.sz[2];
         lo[c] = std::min(lo[c], B.offset);
@@ -572,26 +603,17 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
       P->host_pipeline = true;
     }
   }
-  // longest tiles first within each chunk (cost ~ planes streamed)
-  for (const ChunkRec& c : P->chunks) {
-    auto planes = [&](const TileDev& t) {
-      const UnitDev& u = P->units[t.unit];
-      const BlockDev& B = P->blocks[u.block];
-      return std::min(B.sz[2], 3 + u.k0 + u.nz + kHalo) - std::max(0, 3 + u.k0 - kHalo);
-    };
-    std::stable_sort(P->tiles.begin() + c.tile_begin, P->tiles.begin() + c.tile_begin + c.tile_count,
-                     [&](const TileDev& x, const TileDev& y) { return planes(x) > planes(y); });
-  }
+  order_tiles(P);
   {
-    int sms = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
     const bool mx = precision == B200BSSN_MIXED, adv = P->advective;
-    for (int k = 0; k < 2; ++k) {
-      int per_sm = 0;
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->kind_fn[k], P->deriv_threads, 0);
-      if (o.deriv_ctas_per_sm) per_sm = std::min<int>(per_sm, (int)o.deriv_ctas_per_sm);
-      P->deriv_grid[k] = std::max(1, sms * std::max(1, per_sm));
-    }
+    for (int k = 0; k < 2; ++k)
+      for (int cl = 0; cl < 3; ++cl) {
+        int per_sm = 0;
+        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->kind_fn[k][cl], kItemThreads, 0);
+        // (the option counts CTAs of four warps)
+        if (o.deriv_ctas_per_sm) per_sm = (int)std::min<int64_t>(per_sm, 2 * (int64_t)o.deriv_ctas_per_sm);
+        P->deriv_grid[k][cl] = std::max(1, sms * std::max(1, per_sm));
+      }
     int alg_per_sm = 0;
     if (mx && !adv)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<float, RK_NONE, false>,
@@ -628,14 +650,15 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
       const int nslab = (I2 + kFusedSlab - 1) / kFusedSlab;
       for (int sl = 0; sl < nslab; ++sl) {
         const int k0 = (int)((int64_t)sl * I2 / nslab), k1 = (int)((int64_t)(sl + 1) * I2 / nslab);
-        for (int j0 = 0; j0 < I1; j0 += kTileY)
-          for (int i0 = 0; i0 < I0; i0 += kTileX) {
+        const int cutx = num_cuts(I0, kTileX), cuty = num_cuts(I1, kTileY);
+        for (int ty = 0; ty < cuty; ++ty)
+          for (int tx = 0; tx < cutx; ++tx) {
             FusedTileDev t;
             t.block = (int32_t)b;
-            t.i0 = (int16_t)i0;
-            t.j0 = (int16_t)j0;
-            t.ex = (int16_t)std::min(kTileX, I0 - i0);
-            t.ey = (int16_t)std::min(kTileY, I1 - j0);
+            t.i0 = (int16_t)cut_start(I0, kTileX, tx);
+            t.j0 = (int16_t)cut_start(I1, kTileY, ty);
+            t.ex = (int16_t)(cut_start(I0, kTileX, tx + 1) - t.i0);
+            t.ey = (int16_t)(cut_start(I1, kTileY, ty + 1) - t.j0);
             t.k0 = (int16_t)k0;
             t.nz = (int16_t)(k1 - k0);
             t.pad = 0;
@@ -649,25 +672,23 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
       return B200BSSN_ERR_SIZE_LIMIT;
     }
     P->fsync_words = 4 + 3 * P->ftiles.size() + (size_t)P->nring;
-    int sms = 0, per_sm = 0;
-    cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
+    int per_sm = 0;
     cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, bssn_fused_kernel<RK_NONE>, kFusedThreads,
                                                   kFusedSmemBytes);
     P->fused_grid = std::max(1, sms * std::max(1, per_sm));
   }
 
-  const size_t nb = P->blocks.size() * sizeof(BlockDev), nu = P->units.size() * sizeof(UnitDev),
-               nt = P->tiles.size() * sizeof(TileDev), nr = P->ranges.size() * sizeof(RangeDev);
+  const size_t nb = P->blocks.size() * sizeof(BlockDev), ns = P->slabs.size() * sizeof(SlabDev),
+               nt = P->tiles.size() * sizeof(TileDev),
+               no = P->order.size() * sizeof(int32_t), nr = P->ranges.size() * sizeof(RangeDev);
   auto al = [](size_t x) { return (x + 255) & ~size_t(255); };
-  const size_t total = al(nb) + al(nu) + al(nt) + al(nr);
+  const size_t total = al(nb) + al(ns) + al(nt) + al(no) + al(nr);
   cudaError_t e = cudaMalloc(&P->desc, total);
   const size_t st = precision == B200BSSN_MIXED ? sizeof(float) : sizeof(double);
   const int nbuf = P->chunks.size() > 1 ? 2 : 1;
   for (int b = 0; b < nbuf && e == cudaSuccess; ++b) {
-    // + 512 B: the algebra kernels' copies and prefetches of a slot run are whole
-    // 16-byte chunks or 32-point columns and may read past the last run's end
-    e = cudaMalloc(&P->dscr[b], (size_t)nslots * P->cap * st + 512);
-    if (e == cudaSuccess) e = cudaMalloc(&P->koscr[b], (size_t)kNumVars * P->cap * st + 512);
+    e = cudaMalloc(&P->scr[b], (size_t)nslots * P->cap * st);
+    if (e == cudaSuccess && P->advective) e = cudaMalloc((void**)&P->up[b], (size_t)P->cap);
   }
   if (e == cudaSuccess && P->single_pass) {
     const size_t ntb = al(P->ftiles.size() * sizeof(FusedTileDev));
@@ -680,11 +701,10 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
                      cudaMemcpyHostToDevice);
     }
     const size_t ring_pts = (size_t)P->nring * kFusedSlotPts;
-    if (e == cudaSuccess) e = cudaMalloc(&P->fring_d, ring_pts * kNumDerivs * sizeof(float) + 512);
-    if (e == cudaSuccess) e = cudaMalloc(&P->fring_k, ring_pts * kNumVars * sizeof(float) + 512);
+    if (e == cudaSuccess) e = cudaMalloc(&P->fring, ring_pts * num_slots(false) * sizeof(float));
   }
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&P->ev_fork, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaMalloc((void**)&P->d_counters, 2 * P->chunks.size() * sizeof(int));
+  if (e == cudaSuccess) e = cudaMalloc((void**)&P->d_counters, counter_words(P->chunks.size()) * sizeof(int));
   P->ev_deriv.assign(P->chunks.size(), nullptr);
   P->ev_alg.assign(P->chunks.size(), nullptr);
   P->ev_in.assign(P->chunks.size(), nullptr);
@@ -700,12 +720,14 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   }
   char* base = static_cast<char*>(P->desc);
   P->d_blocks = reinterpret_cast<BlockDev*>(base);
-  P->d_units = reinterpret_cast<UnitDev*>(base + al(nb));
-  P->d_tiles = reinterpret_cast<TileDev*>(base + al(nb) + al(nu));
-  P->d_ranges = reinterpret_cast<RangeDev*>(base + al(nb) + al(nu) + al(nt));
+  P->d_slabs = reinterpret_cast<SlabDev*>(base + al(nb));
+  P->d_tiles = reinterpret_cast<TileDev*>(base + al(nb) + al(ns));
+  P->d_order = reinterpret_cast<int32_t*>(base + al(nb) + al(ns) + al(nt));
+  P->d_ranges = reinterpret_cast<RangeDev*>(base + al(nb) + al(ns) + al(nt) + al(no));
   e = cudaMemcpy(P->d_blocks, P->blocks.data(), nb, cudaMemcpyHostToDevice);
-  if (e == cudaSuccess) e = cudaMemcpy(P->d_units, P->units.data(), nu, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(P->d_slabs, P->slabs.data(), ns, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(P->d_tiles, P->tiles.data(), nt, cudaMemcpyHostToDevice);
+  if (e == cudaSuccess) e = cudaMemcpy(P->d_order, P->order.data(), no, cudaMemcpyHostToDevice);
   if (e == cudaSuccess) e = cudaMemcpy(P->d_ranges, P->ranges.data(), nr, cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     int rc = fail_cuda(ctx, e, "plan upload");
@@ -727,8 +749,8 @@ int b200bssn_plan_destroy(b200bssn_plan* P) {
     cudaStreamSynchronize(P->ctx->s_d2h);
   }
   for (int b = 0; b < 2; ++b) {
-    cudaFree(P->dscr[b]);
-    cudaFree(P->koscr[b]);
+    cudaFree(P->scr[b]);
+    cudaFree(P->up[b]);
   }
   for (cudaEvent_t e : P->ev_deriv)
     if (e) cudaEventDestroy(e);
@@ -740,8 +762,7 @@ int b200bssn_plan_destroy(b200bssn_plan* P) {
   cudaFree(P->d_counters);
   cudaFree(P->d_guard);
   cudaFree(P->fdesc);
-  cudaFree(P->fring_d);
-  cudaFree(P->fring_k);
+  cudaFree(P->fring);
   cudaFree(P->st_u);
   cudaFree(P->st_rhs);
   delete P;
@@ -753,7 +774,12 @@ uint64_t b200bssn_plan_points(const b200bssn_plan* P) { return P ? P->points : 0
 uint32_t b200bssn_plan_launches(const b200bssn_plan* P) {
   if (!P) return 0;
   if (P->single_pass) return 1;                 // the one-pass kernel
-  return (uint32_t)(3 * P->chunks.size());      // two derivative kernels + algebra per chunk
+  uint32_t n = 0;  // per chunk the derivative kernels of its lists that hold tiles, the algebra, the shift signs
+  for (const ChunkRec& c : P->chunks) {
+    n += P->advective ? 2 : 1;
+    for (const int32_t tiles : c.list) n += tiles ? 2 : 0;
+  }
+  return n;
 }
 
 uint32_t b200bssn_plan_single_pass(const b200bssn_plan* P) { return P && P->single_pass ? 1u : 0u; }
@@ -868,7 +894,7 @@ int host_pipelined(b200bssn_plan* P, double* const* rhs, const double* const* u,
   const size_t nch = P->chunks.size();
   const bool preserve = prm->ghost_policy == B200BSSN_GHOSTS_PRESERVE;
   cudaStream_t sin = ctx->s_h2d, s1 = ctx->s_deriv, s2 = ctx->s_alg, sout = ctx->s_d2h;
-  CK(ctx, cudaMemsetAsync(P->d_counters, 0, 2 * nch * sizeof(int), s1));
+  CK(ctx, cudaMemsetAsync(P->d_counters, 0, counter_words(nch) * sizeof(int), s1));
   for (size_t ci = 0; ci < nch; ++ci) {
     const uint64_t a = P->part[ci], b = P->part[ci + 1];
     const size_t nb = (size_t)(b - a) * sizeof(double);
@@ -1075,6 +1101,7 @@ int prepare_block(b200bssn_ctx* ctx, const double* const* u, uint32_t offset, co
     for (int a = 0; a < 3; ++a)
       if (!(pmax[a] > pmin[a])) return B200BSSN_ERR_INVALID_ARGUMENT;
     BlockDev& d = ctx->blk_plan->blocks[0];
+    const bool flags_changed = d.bflag != bflag;
     d.bflag = bflag;
     for (int a = 0; a < 3; ++a) {
       d.pmin[a] = pmin[a];
@@ -1082,6 +1109,13 @@ int prepare_block(b200bssn_ctx* ctx, const double* const* u, uint32_t offset, co
     }
     CK(ctx, cudaMemcpyAsync(ctx->blk_plan->d_blocks, &d, sizeof(BlockDev), cudaMemcpyHostToDevice,
                             ctx->stream));
+    if (flags_changed) {
+      // other tiles have closure rows now
+      b200bssn_plan* P = ctx->blk_plan;
+      order_tiles(P);
+      CK(ctx, cudaMemcpyAsync(P->d_order, P->order.data(), P->order.size() * sizeof(int32_t), cudaMemcpyHostToDevice,
+                              ctx->stream));
+    }
   }
   if (ctx->blk_cap < npad) {
     cudaFree(ctx->blk_u);
@@ -1182,10 +1216,9 @@ ConstraintArgs constraint_args(const b200bssn_plan* P, double* const* con,
   for (int c = 0; c < kNumConstraints; ++c) ca.con[c] = con ? con[c] : nullptr;
   ca.norms = norms;
   ca.blocks = P->d_blocks;
-  ca.units = P->d_units;
+  ca.slabs = P->d_slabs;
   ca.ranges = P->d_ranges;
-  ca.cap = (int32_t)P->cap;
-  ca.nslots = P->advective ? kNumDerivs + 3 * kNumVars : kNumDerivs;
+  ca.nslots = num_slots(P->advective);
   return ca;
 }
 
@@ -1265,29 +1298,28 @@ int b200bssn_debug_block_scratch(b200bssn_ctx* ctx, double* slots, uint64_t npts
   if (P->single_pass || P->chunks.size() != 1 || npts != P->points) return B200BSSN_ERR_INVALID_ARGUMENT;
   CK(ctx, cudaSetDevice(ctx->device));
   CK(ctx, cudaStreamSynchronize(ctx->stream));
-  // the scratch is blocked by 32 points (scr_index): copy it whole, then gather
-  const int ns = P->advective ? kNumDerivs + 3 * kNumVars : kNumDerivs;
+  // copy the scratch whole, then gather
+  const int ns = num_slots(P->advective);
   const size_t nd = (size_t)ns * P->cap;
-  std::vector<double> d(nd), ko((size_t)kNumVars * P->cap);
+  std::vector<double> d(nd);
   if (P->precision == B200BSSN_MIXED) {
     std::vector<float> tmp(nd);
-    CK(ctx, cudaMemcpy(tmp.data(), P->dscr[0], nd * sizeof(float), cudaMemcpyDeviceToHost));
+    CK(ctx, cudaMemcpy(tmp.data(), P->scr[0], nd * sizeof(float), cudaMemcpyDeviceToHost));
     for (size_t k = 0; k < nd; ++k) d[k] = tmp[k];
   } else {
-    CK(ctx, cudaMemcpy(d.data(), P->dscr[0], nd * sizeof(double), cudaMemcpyDeviceToHost));
+    CK(ctx, cudaMemcpy(d.data(), P->scr[0], nd * sizeof(double), cudaMemcpyDeviceToHost));
   }
-  if (P->precision == B200BSSN_MIXED) {
-    std::vector<float> tmp(ko.size());
-    CK(ctx, cudaMemcpy(tmp.data(), P->koscr[0], tmp.size() * sizeof(float), cudaMemcpyDeviceToHost));
-    for (size_t k = 0; k < ko.size(); ++k) ko[k] = tmp[k];
-  } else {
-    CK(ctx, cudaMemcpy(ko.data(), P->koscr[0], ko.size() * sizeof(double), cudaMemcpyDeviceToHost));
-  }
-  auto at = [](int n, int s, uint64_t p) { return ((p >> 5) * n + s) * 32 + (p & 31); };
-  for (int s = 0; s < kNumDerivs; ++s)
-    for (uint64_t p = 0; p < npts; ++p) slots[s * npts + p] = d[at(ns, s, p)];
-  for (int v = 0; v < kNumVars; ++v)
-    for (uint64_t p = 0; p < npts; ++p) slots[(kNumDerivs + v) * npts + p] = ko[at(kNumVars, v, p)];
+  const BlockDev& B = P->blocks[0];
+  const uint64_t I0 = B.sz[0] - 6, I1 = B.sz[1] - 6;
+  for (const RangeDev& rg : P->ranges)
+    for (int k = 0; k < rg.count; ++k)
+      for (int l = 0; l < 32; ++l) {
+        const SlabPoint q = slab_point(B, P->slabs[rg.slab], rg.start + k, l);
+        if (!q.valid) continue;
+        const uint64_t p = (q.i - 3) + I0 * ((q.j - 3) + I1 * (q.k - 3)), at = ((uint64_t)(q.lp >> 5) * ns) * 32 + (q.lp & 31);
+        for (int s = 0; s < kNumDerivs; ++s) slots[s * npts + p] = d[at + 32 * (uint64_t)s];
+        for (int v = 0; v < kNumVars; ++v) slots[(kNumDerivs + v) * npts + p] = d[at + 32 * (uint64_t)(kKoSlot + v)];
+      }
   return B200BSSN_OK;
 }
 

@@ -19,6 +19,7 @@
 #pragma once
 
 #include "plan_types.h"
+#include "rhs_kernels.cuh"
 #include "generated/bssn_constraints_algebra.cuh"
 
 namespace b200bssn {
@@ -30,10 +31,9 @@ struct ConstraintArgs {
   double* con[kNumConstraints];  // all null: fields not written
   double* norms;                 // [nblocks][8] or null
   const BlockDev* blocks;
-  const UnitDev* units;
+  const SlabDev* slabs;
   const RangeDev* ranges;
-  const void* dscr;  // derivative slots, layout scr_index with nslots slots per point
-  int32_t cap;
+  const void* scr;   // derivative slots, layout scr_index with nslots slots per point
   int32_t nslots;
   int32_t range_base;
 };
@@ -45,7 +45,7 @@ struct ConstraintIn {
   int lp;
   __device__ __forceinline__ RT u(int v) const { return (RT)__ldg(a->u[v] + pp); }
   __device__ __forceinline__ RT d(int s) const {
-    return (RT)__ldg(static_cast<const ST*>(a->dscr) + scr_index(a->nslots, s, lp));
+    return (RT)__ldg(static_cast<const ST*>(a->scr) + scr_index(a->nslots, s, lp));
   }
 };
 
@@ -65,38 +65,28 @@ template <typename RT, typename ST>
 __global__ void __launch_bounds__(kAlgebraThreads)
 bssn_constraints_kernel(const __grid_constant__ ConstraintArgs a) {
   const RangeDev rg = a.ranges[a.range_base + blockIdx.x];
-  const UnitDev un = a.units[rg.unit];
-  const BlockDev& B = a.blocks[un.block];
-  const bool active = (int)threadIdx.x < rg.count;
-  if (sizeof(ST) == 8 && rg.count > 0) {
+  const SlabDev slab = a.slabs[rg.slab];
+  const BlockDev& B = a.blocks[slab.block];
+  const int task = threadIdx.x / 32;
+  const SlabPoint p = slab_point(B, slab, rg.start + min(task, rg.count - 1), threadIdx.x % 32);
+  const bool active = task < rg.count && p.valid;
+  if (sizeof(ST) == 8) {
     // FP64 (latency bound at 255 registers): pull the run's scratch into L2 first, so
-    // the per-point loads below hit L2; its 32-point blocks are one contiguous run
-    // (16-byte aligned), prefetched in pieces of at most 4 KB.  (MIXED, closer to the
-    // DRAM bound, lost 3 % to the extra instructions.)
-    const int lp0 = (int)un.sbase + rg.start;
-    const int b0 = lp0 >> 5, nblk = ((lp0 + rg.count - 1) >> 5) - b0 + 1;
-    const char* pd = reinterpret_cast<const char*>(static_cast<const ST*>(a.dscr) + (size_t)b0 * a.nslots * 32);
-    const uint32_t td = (uint32_t)nblk * (uint32_t)a.nslots * 32u * (uint32_t)sizeof(ST);
-    const int npc = (int)((td + 4095u) / 4096u);
-    for (int k = threadIdx.x; k < npc; k += kAlgebraThreads)
-      asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(pd + 4096u * (uint32_t)k),
-                   "r"(min(4096u, td - 4096u * (uint32_t)k))
-                   : "memory");
+    // the per-point loads below hit L2: one sector per group and derivative slot that the
+    // constraints read.  (MIXED, closer to the DRAM bound, lost 3 % to the extra
+    // instructions.)
+    const ST* const own = static_cast<const ST*>(a.scr) + scr_index(a.nslots, 0, p.lp - (int)(threadIdx.x % kGroup));
+    for (int s = threadIdx.x % kGroup; s < kNumDerivs; s += kGroup) prefetch_l2(own + s * 32);
   }
   double sq[kNumConstraints] = {0.0, 0.0, 0.0, 0.0};
   double mx[kNumConstraints] = {0.0, 0.0, 0.0, 0.0};
   if (active) {
-    const int nx = B.sz[0], ny = B.sz[1];
-    const int I0 = nx - 6, I1 = ny - 6;
-    const int lpu = rg.start + threadIdx.x;
-    const int lx = lpu % I0, rr = lpu / I0, ly = rr % I1, lz = rr / I1;
-    const int64_t pp =
-        B.offset + (lx + 3) + (int64_t)nx * ((ly + 3) + (int64_t)ny * (lz + 3 + un.k0));
+    const int64_t pp = B.offset + p.i + (int64_t)B.sz[0] * (p.j + (int64_t)B.sz[1] * p.k);
     if (sizeof(ST) == 8) {
 #pragma unroll
-      for (int v = 0; v < kNumVars; ++v) asm volatile("prefetch.global.L2 [%0];" ::"l"(a.u[v] + pp));
+      for (int v = 0; v < kNumVars; ++v) prefetch_l2(a.u[v] + pp);
     }
-    ConstraintIn<RT, ST> in{&a, pp, (int)un.sbase + lpu};
+    ConstraintIn<RT, ST> in{&a, pp, p.lp};
     ConstraintSink<RT> sink;
     bssn_constraints_algebra<RT>(in, sink);
 #pragma unroll
@@ -132,10 +122,10 @@ bssn_constraints_kernel(const __grid_constant__ ConstraintArgs a) {
     const int c = threadIdx.x;
     double r = s_red[0][c];
     for (int k = 1; k < kAlgebraThreads / 32; ++k) {
-      const double t = s_red[k][c];
-      r = c < kNumConstraints ? r + t : ((t > r || t != t) ? t : r);
+      const double w = s_red[k][c];
+      r = c < kNumConstraints ? r + w : ((w > r || w != w) ? w : r);
     }
-    double* dst = a.norms + (size_t)un.block * (2 * kNumConstraints) + c;
+    double* dst = a.norms + (size_t)slab.block * (2 * kNumConstraints) + c;
     if (c < kNumConstraints)
       atomicAdd(dst, r);
     else

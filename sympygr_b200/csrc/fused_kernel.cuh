@@ -8,11 +8,11 @@
 // Work units (plan order, see b200bssn.cu):
 //   tile-slab T  a 16x8 column tile of a block over a z-slab of at most kFusedSlab
 //                interior planes; it owns ring slot T % nring while in flight
-//   item (T, v)  the derivative stage of variable v on tile-slab T (derive_item, the
-//                same streaming stencil as the two-pass kernels), written into the
-//                slot in the blocked layout of 32-point runs: point (tx, ty, z) of the
-//                tile is lp = slot * kFusedSlotPts + tx + 16 ty + 128 z
-//   planes of T  the algebra of plane z of tile-slab T: warp w takes rows 2w, 2w+1
+//   item (T, g)  the derivative stage of two variables on tile-slab T, one per pair of
+//                warps (derive_item, the same streaming stencil as the two-pass kernels),
+//                written into the slot in the plans' scratch layout: point (tx, ty, z) of
+//                the tile is lp = slot * kFusedSlotPts + tx + row_off(ty) + 128 z
+//   planes of T  the algebra of plane z of tile-slab T: warp w takes block w of the plane
 //                (one 32-point run), copies its 138 slots into shared memory and runs
 //                the generated algebra, the Sommerfeld faces and the KO term
 //                (algebra_point_at), storing the RHS or an RK4 stage update; a claim
@@ -21,7 +21,7 @@
 // Scheduling (warp 0 of each CTA, all 32 lanes together):
 //   * algebra first: the lanes look at the next 32 tile-slabs from the algebra hint
 //     (the first tile-slab whose algebra is not all claimed) at once; a tile-slab whose
-//     24 items are done hands out its planes kFusedPlanes at a time through its own
+//     12 items are done hands out its planes kFusedPlanes at a time through its own
 //     fetch-and-add counter, so no single counter serialises the claims;
 //   * else the next item, by fetch-and-add on the item counter; if its tile-slab's
 //     ring slot is not free yet (the tile-slab nring earlier still has algebra
@@ -49,10 +49,14 @@ constexpr int kFusedMinBlocks = 3;                              // CTAs per SM (
 constexpr unsigned long long kFusedWaitNs = 2000000000ull;      // 2 s per wait, then an error
 constexpr size_t kFusedStageBytes = (size_t)kNumDerivs * kStageW * sizeof(float);  // per warp
 constexpr size_t kFusedSmemBytes = 4 * kFusedStageBytes;        // 70,656 B (derivative buffers alias it)
-static_assert(4 * kPlane * sizeof(double) + 2 * kDxRows * kTileX * sizeof(double) +
-                      (kHalo + 1) * kDerivThreads * sizeof(double) <= kFusedSmemBytes,
-              "the derivative item's buffers fit in the algebra staging area");
-static_assert(kFusedThreads == kDerivThreads, "one CTA shape for both roles");
+constexpr int kFusedItemVars = kFusedThreads / kItemThreads;    // variables of an item
+constexpr int kFusedItems = kNumVars / kFusedItemVars;          // items of a tile-slab
+union DerivSmemAny {
+  DerivSmem<true> dd;
+  DerivSmem<false> nd;
+};
+static_assert(kFusedItemVars * sizeof(DerivSmemAny) <= kFusedSmemBytes, "the derivative items' buffers fit in the algebra staging area");
+static_assert(kFusedSlotPts == kTilePlane * kFusedSlab, "a ring slot is a tile of the scratch layout");
 
 // Device words of one evaluation, zeroed before the launch:
 //   [0] next item, [1] algebra hint, [2] error (1: a wait timed out), [3] unused,
@@ -60,7 +64,7 @@ static_assert(kFusedThreads == kDerivThreads, "one CTA shape for both roles");
 //   used[ntiles] (planes whose algebra is finished), gen[nring] (slot s is free for
 //   tile-slab T when gen[s] == T / nring)
 struct FusedArgs {
-  DerivArgs d;        // state, blocks; dscr/koscr = the ring (MIXED: float)
+  DerivArgs d;        // state, blocks; scr = the ring (MIXED: float)
   AlgebraArgs a;      // state, RHS or RK4 stage, parameters
   const FusedTileDev* tiles;
   int32_t ntiles, nring;
@@ -93,7 +97,7 @@ __device__ __forceinline__ int fused_schedule(const FusedArgs& f, int& pending, 
   const int* const done = f.sync + 4;
   int* const claimed = f.sync + 4 + f.ntiles;
   const int* const gen = f.sync + 4 + 3 * f.ntiles;
-  const int nitems = f.ntiles * kNumVars;
+  const int nitems = f.ntiles * kFusedItems;
   unsigned long long t0 = 0;
   unsigned sleep = 32;
   for (;;) {
@@ -108,8 +112,8 @@ __device__ __forceinline__ int fused_schedule(const FusedArgs& f, int& pending, 
       dn = ld_relaxed(done + T);
       cl = ld_relaxed(claimed + T);
     }
-    const bool ready = inwin && dn == kNumVars && cl < nz;
-    const unsigned exhausted = __ballot_sync(0xffffffffu, inwin && dn == kNumVars && cl >= nz);
+    const bool ready = inwin && dn == kFusedItems && cl < nz;
+    const unsigned exhausted = __ballot_sync(0xffffffffu, inwin && dn == kFusedItems && cl >= nz);
     const int adv = exhausted == 0xffffffffu ? 32 : __ffs(~exhausted) - 1;  // leading fully claimed tile-slabs
     if (adv > 0 && lane == 0) atomicMax(hint, h + adv);
     unsigned rmask = __ballot_sync(0xffffffffu, ready);
@@ -136,7 +140,7 @@ __device__ __forceinline__ int fused_schedule(const FusedArgs& f, int& pending, 
       if (d < nitems) pending = d;
     }
     if (pending >= 0) {
-      const int Tp = pending / kNumVars;
+      const int Tp = pending / kFusedItems;
       if (ld_relaxed(gen + Tp % f.nring) == Tp / f.nring) {
         __threadfence();  // the slot's previous readers are done before it is rewritten
         *idx = pending;
@@ -171,16 +175,17 @@ template <int MODE>
 __global__ void __launch_bounds__(kFusedThreads, kFusedMinBlocks)
 bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
   extern __shared__ __align__(16) unsigned char smem[];
-  __shared__ LineScales s_sc[3];
   __shared__ int s_role, s_idx, s_p0, s_np;
-  double* s_plane = reinterpret_cast<double*>(smem);
-  double* s_dxp = reinterpret_cast<double*>(smem + 4 * kPlane * sizeof(double));
-  double* s_kq = s_dxp + 2 * kDxRows * kTileX;
+  __shared__ ClosureRow s_closure[6];
+  __shared__ ClosureValues s_fix[kFusedItemVars];
+  load_closure_rows(s_closure);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* const done = f.sync + 4;
   int* const used = f.sync + 4 + 2 * f.ntiles;
   int* const gen = f.sync + 4 + 3 * f.ntiles;
   int pending = -1;  // warp 0: the item this CTA holds
+  const int half = threadIdx.x / kItemThreads;  // this thread's variable of an item
+  DerivSmemAny& S = reinterpret_cast<DerivSmemAny*>(smem)[half];
 
   for (;;) {
     if (warp == 0) {
@@ -197,22 +202,21 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
     const int role = s_role, idx = s_idx;
     if (role == FR_EXIT) break;
     if (role == FR_ITEM) {
-      const int T = idx / kNumVars, v = idx % kNumVars;
+      const int T = idx / kFusedItems, v = kFusedItemVars * (idx % kFusedItems) + half;
       const FusedTileDev ft = f.tiles[T];
-      const UnitDev un{ft.block, ft.k0, ft.nz, 0, 0};
-      const TileDev t{0, ft.i0, ft.j0, ft.ex, ft.ey};
-      const ScratchMap sm{(T % f.nring) * kFusedSlotPts, kTileX, kTileX * kTileY};
-      const bool cl = item_has_closure(f.d.blocks[ft.block], un, t);
+      const TileDev t{ft.block, 0, ft.k0, ft.nz, ft.i0, ft.j0, ft.ex, ft.ey};
+      const ScratchMap sm{(T % f.nring) * kFusedSlotPts, 0, 0};
+      const bool cl = tile_closure(f.d.blocks[ft.block], t) != kClosureNone;
       if (dd_index(v) >= 0) {
         if (cl)
-          derive_item<float, true, false, true>(f.d, un, t, sm, v, s_plane, s_dxp, s_kq, s_sc);
+          derive_item<float, true, false, kClosureXY, true>(f.d, f.d.blocks[ft.block], t, sm, v, S.dd, s_closure, s_fix + half, 1 + half);
         else
-          derive_item<float, true, false, false>(f.d, un, t, sm, v, s_plane, s_dxp, s_kq, s_sc);
+          derive_item<float, true, false, kClosureNone, true>(f.d, f.d.blocks[ft.block], t, sm, v, S.dd, s_closure, s_fix + half, 1 + half);
       } else {
         if (cl)
-          derive_item<float, false, false, true>(f.d, un, t, sm, v, s_plane, s_dxp, s_kq, s_sc);
+          derive_item<float, false, false, kClosureXY, true>(f.d, f.d.blocks[ft.block], t, sm, v, S.nd, s_closure, s_fix + half, 1 + half);
         else
-          derive_item<float, false, false, false>(f.d, un, t, sm, v, s_plane, s_dxp, s_kq, s_sc);
+          derive_item<float, false, false, kClosureNone, true>(f.d, f.d.blocks[ft.block], t, sm, v, S.nd, s_closure, s_fix + half, 1 + half);
       }
       __threadfence();  // this thread's slot writes, before the done count
       __syncthreads();
@@ -221,14 +225,15 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
       const int T = idx, pz0 = s_p0, npl = s_np;
       const FusedTileDev ft = f.tiles[T];
       const BlockDev& B = f.a.blocks[ft.block];
-      const int tx = lane & 15, ty = 2 * warp + (lane >> 4);
-      const bool any = 2 * warp < ft.ey;
+      // block `warp` of a plane holds rows y and y + 2 (row_off)
+      const int y0 = (warp & 1) + 4 * (warp >> 1), tx = lane & 15, ty = y0 + 2 * (lane >> 4);
+      const bool any = y0 < ft.ey;
       const bool valid = tx < ft.ex && ty < ft.ey;
       float* sd = reinterpret_cast<float*>(smem + warp * kFusedStageBytes);
       for (int z = pz0; any && z < pz0 + npl; ++z) {
         const int run = (T % f.nring) * (kFusedSlotPts / 32) + z * 4 + warp;  // 32-point run in the ring
-        const float* gd = static_cast<const float*>(f.d.dscr) + (size_t)run * kNumDerivs * 32;
-        const float* gk = static_cast<const float*>(f.d.koscr) + (size_t)run * kNumVars * 32;
+        const float* gd = static_cast<const float*>(f.d.scr) + (size_t)run * num_slots(false) * 32;
+        const float* gk = gd + kKoSlot * 32;
         const int i = 3 + ft.i0 + tx, j = 3 + ft.j0 + ty, k = 3 + ft.k0 + z;
         if (valid) {
           const int64_t pp = B.offset + i + (int64_t)B.sz[0] * (j + (int64_t)B.sz[1] * k);
@@ -246,7 +251,7 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
         constexpr int ND = (int)(kFusedStageBytes / 16);
 #pragma unroll 6
         for (int q = lane; q < ND; q += 32)
-          cp_async16(reinterpret_cast<char*>(sd) + 16 * q, reinterpret_cast<const char*>(gd) + 16 * q);
+          cp_async16(static_cast<uint32_t>(__cvta_generic_to_shared(sd)) + 16u * q, reinterpret_cast<uint64_t>(gd) + 16u * q);
         cp_async_commit();
         cp_async_wait<0>();
         __syncwarp();

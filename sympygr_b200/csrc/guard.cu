@@ -21,22 +21,21 @@ struct GuardArgs {
   const double* a[kNumVars];
   int32_t narrays;
   const BlockDev* blocks;
-  const UnitDev* units;
+  const SlabDev* slabs;
   const RangeDev* ranges;
   unsigned long long* first_bad;
 };
 
 __global__ void __launch_bounds__(kAlgebraThreads) finite_guard_kernel(const __grid_constant__ GuardArgs g) {
   const RangeDev rg = g.ranges[blockIdx.x];
-  if ((int)threadIdx.x >= rg.count) return;
-  const UnitDev un = g.units[rg.unit];
-  const BlockDev& B = g.blocks[un.block];
-  const int nx = B.sz[0], ny = B.sz[1];
-  const int I0 = nx - 6, I1 = ny - 6;
-  const int lpu = rg.start + threadIdx.x;
-  const int lx = lpu % I0, rr = lpu / I0, ly = rr % I1, lz = rr / I1;
+  const int task = threadIdx.x / 32;
+  if (task >= rg.count) return;
+  const SlabDev s = g.slabs[rg.slab];
+  const BlockDev& B = g.blocks[s.block];
+  const SlabPoint p = slab_point(B, s, rg.start + task, threadIdx.x % 32);
+  if (!p.valid) return;
   const unsigned long long pp =
-      B.offset + (lx + 3) + (unsigned long long)nx * ((ly + 3) + (unsigned long long)ny * (lz + 3 + un.k0));
+      B.offset + p.i + (unsigned long long)B.sz[0] * (p.j + (unsigned long long)B.sz[1] * p.k);
   bool bad = false;
   for (int v = 0; v < g.narrays; ++v) bad |= !isfinite(__ldg(g.a[v] + pp));
   if (bad) atomicMin(g.first_bad, pp);
@@ -61,7 +60,7 @@ int b200bssn_check_finite(b200bssn_plan* P, const double* const* arrays, uint32_
   for (uint32_t v = 0; v < narrays; ++v) g.a[v] = arrays[v];
   g.narrays = (int32_t)narrays;
   g.blocks = P->d_blocks;
-  g.units = P->d_units;
+  g.slabs = P->d_slabs;
   g.ranges = P->d_ranges;
   g.first_bad = P->d_guard;
   CK(ctx, cudaMemsetAsync(P->d_guard, 0xff, sizeof(unsigned long long), s));

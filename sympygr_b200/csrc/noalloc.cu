@@ -5,34 +5,32 @@
 // pool allocator at start-up (so a library cudaMalloc would fail or fragment that
 // pool), and a time-step loop that must not call cudaMalloc/cudaFree because they
 // can synchronise the whole device.  Such callers own the input and output arrays;
-// the only other memory this path needs -- the derivative scratch and the work
-// descriptors -- lives in one fixed array below, reserved when the library is
-// loaded and held by every GPU that loads it until the process exits.
+// the only other memory this path needs -- the derivative scratch -- lives in one fixed
+// array below, reserved when the library is loaded and held by every GPU that loads it
+// until the process exits; the work descriptors are kernel arguments.
 //
 // Limits and sharing:
 //  * at most kNoallocMaxPoints interior points per call (a block with a 32^3
 //    interior, i.e. 38^3 padded, is the largest cube that fits); larger blocks
 //    are rejected with B200BSSN_ERR_SIZE_LIMIT before anything is launched;
 //  * every call on a device uses the same array, which keeps whatever the last
-//    call left in it.  Each call rewrites every word it later reads (descriptors
-//    first, then every derivative slot of every interior point), so nothing has
-//    to start at zero -- but two calls whose work overlaps on the GPU (different
+//    call left in it.  Each call rewrites every word it later reads (every
+//    derivative slot of every interior point), so nothing has to start at zero -- but two calls whose work overlaps on the GPU (different
 //    streams, or host threads racing) overwrite each other's scratch and give
 //    wrong results.  Serialise calls per device;
 //  * the first call on each device looks up the array's device address with
-//    cudaGetSymbolAddress, sets the derivative kernel's shared-memory limit and
-//    reads its occupancy, with that device current; make that first call before any
+//    cudaGetSymbolAddress, with that device current; make that first call before any
 //    stream capture.  The address is kept for the life of the process, so calls after
 //    a cudaDeviceReset of that device (which reloads the library's device code at a
 //    new address) are not supported.
 //
-// The derivative kernel here is the combined one over all 24 variables
-// (bssn_derivs_kernel), which only this entry point launches; the plans use the two
-// per-kind kernels.
+// The derivatives come from the plans' kernels in a form that numbers scratch points
+// densely, tile after tile: the array has no room for the plans' padding.  Every tile takes
+// the form with closure rows when the block has a flagged face.
 #include <cuda_runtime.h>
 
+#include <algorithm>
 #include <cstring>
-
 #include <mutex>
 
 #include "b200bssn.h"
@@ -43,112 +41,120 @@ using namespace b200bssn;
 namespace {
 
 constexpr int64_t kNoallocMaxPoints = B200BSSN_NOALLOC_MAX_POINTS;
-constexpr int kNoallocMaxUnits = 1024;
-constexpr int kNoallocMaxTiles = 4096;
-constexpr int kNoallocMaxRanges = 2048;
 constexpr int kMaxDevices = 64;
-constexpr int kNoallocSlab = 48;  // z-slab depth of this path's work units
+constexpr int kNoallocSlab = 48;  // greatest z-slab depth of this path
 
-// byte layout of the fixed array (each part 256-byte aligned)
-constexpr size_t al256(size_t x) { return (x + 255) & ~size_t(255); }
-constexpr size_t kOffCounter = 0;
-constexpr size_t kOffBlock = kOffCounter + 256;
-constexpr size_t kOffUnits = kOffBlock + al256(sizeof(BlockDev));
-constexpr size_t kOffTiles = kOffUnits + al256(sizeof(UnitDev) * kNoallocMaxUnits);
-constexpr size_t kOffRanges = kOffTiles + al256(sizeof(TileDev) * kNoallocMaxTiles);
-constexpr size_t kOffDeriv = kOffRanges + al256(sizeof(RangeDev) * kNoallocMaxRanges);
-constexpr size_t kOffKo = kOffDeriv + al256(sizeof(double) * kNumDerivs * kNoallocMaxPoints);
-// + 256: the algebra kernel's L2 prefetch of a slot run rounds its size up to 16 bytes
-constexpr size_t kNoallocBytes = kOffKo + al256(sizeof(double) * kNumVars * kNoallocMaxPoints) + 256;
+// the derivative scratch
+constexpr size_t kNoallocBytes = sizeof(double) * num_slots(false) * kNoallocMaxPoints;
 
 static __device__ __align__(256) unsigned char g_noalloc_scratch[kNoallocBytes];
 
-// Per-device address of g_noalloc_scratch (host-side handle -> device address) and
-// the resident CTA count of the persistent derivative kernel, per precision.
+// Per-device address of g_noalloc_scratch (host-side handle -> device address) and the
+// SM count.
+struct DeviceSetup {
+  void* addr = nullptr;
+  int sms = 0;
+};
 std::mutex g_setup_mutex;
-void* g_scratch_addr[kMaxDevices] = {};
-int g_deriv_grid[kMaxDevices][2] = {};  // [dev][0: FP64, 1: MIXED]
+DeviceSetup g_setup[kMaxDevices];
 
-int setup_device(int dev, void** addr, int* grid64, int* grid32) {
+int setup_device(int dev, DeviceSetup* out) {
   std::lock_guard<std::mutex> lock(g_setup_mutex);
-  if (g_scratch_addr[dev]) {
-    *addr = g_scratch_addr[dev];
-    *grid64 = g_deriv_grid[dev][0];
-    *grid32 = g_deriv_grid[dev][1];
-    return B200BSSN_OK;
+  DeviceSetup& d = g_setup[dev];
+  if (!d.addr) {
+    void* p = nullptr;
+    int sms = 0;
+    if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess || sms <= 0) {
+      cudaGetLastError();
+      return B200BSSN_ERR_CUDA;
+    }
+    d.sms = sms;
+    d.addr = p;
   }
-  void* p = nullptr;
-  if (cudaGetSymbolAddress(&p, g_noalloc_scratch) != cudaSuccess || p == nullptr) {
-    cudaGetLastError();
-    return B200BSSN_ERR_CUDA;
-  }
-  if (cudaFuncSetAttribute(bssn_derivs_kernel<double>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kDerivSmemBytes) != cudaSuccess ||
-      cudaFuncSetAttribute(bssn_derivs_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                           (int)kDerivSmemBytes) != cudaSuccess) {
-    cudaGetLastError();
-    return B200BSSN_ERR_CUDA;
-  }
-  // the derivative kernel is persistent (each CTA pulls items from the work counter),
-  // so its grid is the CTAs that fit on the GPU at once, as the plans size it
-  int sms = 0, occ64 = 0, occ32 = 0;
-  if (cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ64, bssn_derivs_kernel<double>, kDerivThreads,
-                                                    kDerivSmemBytes) != cudaSuccess ||
-      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ32, bssn_derivs_kernel<float>, kDerivThreads,
-                                                    kDerivSmemBytes) != cudaSuccess ||
-      sms <= 0 || occ64 <= 0 || occ32 <= 0) {
-    cudaGetLastError();
-    return B200BSSN_ERR_CUDA;
-  }
-  g_deriv_grid[dev][0] = sms * occ64;
-  g_deriv_grid[dev][1] = sms * occ32;
-  g_scratch_addr[dev] = p;
-  *addr = p;
-  *grid64 = g_deriv_grid[dev][0];
-  *grid32 = g_deriv_grid[dev][1];
+  *out = d;
   return B200BSSN_OK;
 }
 
-// Writes the work descriptors of one block (z-slab units of kNoallocSlab planes, x-y
-// tiles, runs of kAlgebraThreads points) -- the layout b200bssn_plan_create
-// builds on the host -- straight into the fixed array.
-__global__ void noalloc_describe(BlockDev blk, BlockDev* blk_out, int* counter, UnitDev* units,
-                                 TileDev* tiles, RangeDev* ranges, int n_units, int tiles_x,
-                                 int tiles_y, int ranges_per_unit_max) {
-  if (blockIdx.x == 0 && threadIdx.x == 0) {
-    *blk_out = blk;
-    *counter = 0;  // work counter of the derivative kernel
+// The one block of a call, as kernel arguments: its tiles are numbered slab by slab, and
+// their scratch points lie densely, tile after tile.
+struct NoallocGeom {
+  BlockDev block;
+  int tiles_x, tiles_y, slabs;
+  int runs;  // runs of kAlgebraThreads points per tile, of the largest one
+};
+__device__ __forceinline__ TileDev noalloc_tile(const NoallocGeom& g, int k) {
+  const int I0 = g.block.sz[0] - 6, I1 = g.block.sz[1] - 6, I2 = g.block.sz[2] - 6;
+  const int u = k / (g.tiles_x * g.tiles_y), ty = k / g.tiles_x % g.tiles_y, tx = k % g.tiles_x;
+  TileDev t;
+  t.block = 0;
+  t.k0 = u * I2 / g.slabs;  // near-equal slabs (never below three planes)
+  t.nz = (u + 1) * I2 / g.slabs - t.k0;
+  t.i0 = (int16_t)cut_start(I0, kTileX, tx);
+  t.j0 = (int16_t)cut_start(I1, kTileY, ty);
+  t.ex = (int16_t)(cut_start(I0, kTileX, tx + 1) - t.i0);
+  t.ey = (int16_t)(cut_start(I1, kTileY, ty + 1) - t.j0);
+  t.sbase = I0 * I1 * t.k0 + t.nz * (I0 * t.j0 + t.i0 * t.ey);  // points of the tiles before
+  return t;
+}
+
+// One (tile, variable) item per CTA.
+template <typename ST, bool DD, int CLOSURE>
+__global__ void __launch_bounds__(kItemThreads, kind_ctas_per_sm(DD, false, CLOSURE))
+noalloc_derivs(const __grid_constant__ DerivArgs a, const __grid_constant__ NoallocGeom g) {
+  constexpr int NV = kKindVars[DD];
+  __shared__ DerivSmem<DD> S;
+  __shared__ ClosureRow s_closure[CLOSURE == kClosureXY ? 6 : 1];
+  __shared__ __align__(8) unsigned char s_fix[CLOSURE == kClosureXY ? sizeof(ClosureValues) : 8];
+  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  if (CLOSURE == kClosureXY) {
+    load_closure_rows(s_closure);
+    __syncthreads();
   }
-  const int I0 = blk.sz[0] - 6, I1 = blk.sz[1] - 6, I2 = blk.sz[2] - 6;
-  const int tiles_per_unit = tiles_x * tiles_y;
-  for (int u = blockIdx.x * blockDim.x + threadIdx.x; u < n_units; u += gridDim.x * blockDim.x) {
-    UnitDev d;
-    d.block = 0;
-    d.k0 = u * kNoallocSlab;
-    d.nz = min(kNoallocSlab, I2 - d.k0);
-    d.pad = 0;
-    d.sbase = (int64_t)I0 * I1 * d.k0;
-    units[u] = d;
-    const int np = I0 * I1 * d.nz;
-    for (int r = 0; r < ranges_per_unit_max; ++r) {
-      RangeDev g;
-      g.unit = u;
-      g.start = r * kAlgebraThreads;
-      g.count = max(0, min(kAlgebraThreads, np - g.start));
-      ranges[u * ranges_per_unit_max + r] = g;
-    }
-    for (int t = 0; t < tiles_per_unit; ++t) {
-      TileDev td;
-      td.unit = u;
-      const int tx = t % tiles_x, ty = t / tiles_x;
-      td.i0 = (int16_t)(tx * kTileX);
-      td.j0 = (int16_t)(ty * kTileY);
-      td.ex = (int16_t)min(kTileX, I0 - tx * kTileX);
-      td.ey = (int16_t)min(kTileY, I1 - ty * kTileY);
-      tiles[u * tiles_per_unit + t] = td;
-    }
-  }
+  const TileDev t = noalloc_tile(g, blockIdx.x / NV);
+  const ScratchMap sm{t.sbase, t.ex, t.ex * t.ey};
+  derive_item<ST, DD, false, CLOSURE, false>(a, g.block, t, sm, kind_var(DD, blockIdx.x % NV), S, s_closure,
+                                             reinterpret_cast<ClosureValues*>(s_fix), 1);
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+template <typename ST>
+const void* derivs_kernel(bool dd, bool closure) {
+  if (dd)
+    return closure ? (const void*)noalloc_derivs<ST, true, kClosureXY> : (const void*)noalloc_derivs<ST, true, kClosureNone>;
+  return closure ? (const void*)noalloc_derivs<ST, false, kClosureXY> : (const void*)noalloc_derivs<ST, false, kClosureNone>;
+}
+
+template <typename ST>
+struct GlobalScratch {
+  const ST* d;       // slot 0 of the point
+  __device__ __forceinline__ ST dv(int s) const { return __ldg(d + s * 32); }
+  __device__ __forceinline__ double kov(int v) const { return (double)__ldg(d + (kKoSlot + v) * 32); }
+};
+
+// The algebra: one CTA per run of up to 128 points of a tile, one thread per point, inputs
+// loaded from global memory as the generated code needs them.
+template <typename ST>
+__global__ void __launch_bounds__(kAlgebraThreads, 2)
+noalloc_algebra(const __grid_constant__ AlgebraArgs a, const __grid_constant__ NoallocGeom g) {
+  constexpr int NS = num_slots(false);
+  const int tile = blockIdx.x / g.runs, start = (blockIdx.x - tile * g.runs) * kAlgebraThreads;
+  const TileDev t = noalloc_tile(g, tile);
+  const int count = min(kAlgebraThreads, t.ex * t.ey * t.nz - start);
+  if (count <= 0) return;
+  // pull this CTA's scratch into L2 first, so the per-point loads below hit L2 instead of
+  // waiting on DRAM: the 32-point blocks its points fall in are one contiguous run (every
+  // block starts on a 16-byte boundary), in pieces of at most 4 KB
+  const int lp0 = t.sbase + start;
+  const int b0 = lp0 >> 5, nblk = ((lp0 + count - 1) >> 5) - b0 + 1;
+  const char* pd = reinterpret_cast<const char*>(static_cast<const ST*>(a.scr) + (size_t)b0 * NS * 32);
+  const uint32_t td = (uint32_t)nblk * NS * 32 * sizeof(ST);
+  for (uint32_t off = 4096u * threadIdx.x; off < td; off += 4096u * kAlgebraThreads)
+    prefetch_l2_bulk(pd + off, min(4096u, td - off));
+  if ((int)threadIdx.x >= count) return;
+  const int lp = start + threadIdx.x, r = lp / t.ex, z = r / t.ey;
+  const GlobalScratch<ST> src{static_cast<const ST*>(a.scr) + scr_index<NS>(0, t.sbase + lp)};
+  algebra_point_at<ST, RK_NONE>(a, g.block, 3 + t.i0 + (lp - r * t.ex), 3 + t.j0 + (r - z * t.ey), 3 + t.k0 + z, src);
 }
 
 }  // namespace
@@ -168,11 +174,12 @@ extern "C" int b200bssn_rhs_noalloc(double* const* rhs_dev, const double* const*
   if (block->bflag >> 6) return B200BSSN_ERR_INVALID_ARGUMENT;
   const int64_t I0 = block->sz[0] - 6, I1 = block->sz[1] - 6, I2 = block->sz[2] - 6;
   const int64_t npts = I0 * I1 * I2;
-  const int64_t n_units = (I2 + kNoallocSlab - 1) / kNoallocSlab;
   const int64_t tiles_x = (I0 + kTileX - 1) / kTileX, tiles_y = (I1 + kTileY - 1) / kTileY;
-  const int64_t rpu = (I0 * I1 * kNoallocSlab + kAlgebraThreads - 1) / kAlgebraThreads;
-  if (npts > kNoallocMaxPoints || n_units > kNoallocMaxUnits ||
-      n_units * tiles_x * tiles_y > kNoallocMaxTiles || n_units * rpu > kNoallocMaxRanges)
+  const auto pieces = [](int64_t n, int64_t size) { return (n + size - 1) / size; };
+  // (the limits of descriptor arrays that are gone; kept so that the same blocks are refused)
+  const int64_t fewest = pieces(I2, kNoallocSlab);
+  if (npts > kNoallocMaxPoints || fewest > 1024 || fewest * tiles_x * tiles_y > 4096 ||
+      fewest * pieces(I0 * I1 * kNoallocSlab, kAlgebraThreads) > 2048)
     return B200BSSN_ERR_SIZE_LIMIT;
 
   int dev = 0;
@@ -180,17 +187,16 @@ extern "C" int b200bssn_rhs_noalloc(double* const* rhs_dev, const double* const*
     cudaGetLastError();
     return B200BSSN_ERR_NO_DEVICE;
   }
-  void* base = nullptr;
-  int grid64 = 0, grid32 = 0;
-  int rc = setup_device(dev, &base, &grid64, &grid32);
+  DeviceSetup setup;
+  const int rc = setup_device(dev, &setup);
   if (rc != B200BSSN_OK) return rc;
-  char* b = static_cast<char*>(base);
-  UnitDev* units = reinterpret_cast<UnitDev*>(b + kOffUnits);
-  TileDev* tiles = reinterpret_cast<TileDev*>(b + kOffTiles);
-  RangeDev* ranges = reinterpret_cast<RangeDev*>(b + kOffRanges);
-  BlockDev* bd = reinterpret_cast<BlockDev*>(b + kOffBlock);
-
-  BlockDev blk;
+  // as many slabs as fill the GPU with one wave of the 11 variables with second derivatives (6
+  // CTAs per SM), but none below three planes (38^3: ten slabs)
+  const int64_t columns = tiles_x * tiles_y;
+  const int64_t slabs = std::max(fewest, std::min<int64_t>(I2 / 3, 6 * setup.sms / (columns * kKindVars[1])));
+  const int64_t n_tiles = slabs * columns;
+  NoallocGeom g;
+  BlockDev& blk = g.block;
   blk.offset = block->offset;
   blk.bflag = block->bflag;
   for (int a = 0; a < 3; ++a) {
@@ -199,12 +205,10 @@ extern "C" int b200bssn_rhs_noalloc(double* const* rhs_dev, const double* const*
     blk.h[a] = (block->pmax[a] - block->pmin[a]) / (block->sz[a] - 1);  // rhs.cpp:144-146
   }
   cudaStream_t s = static_cast<cudaStream_t>(stream);
-  // the block descriptor travels as a kernel argument and the kernel stores it,
-  // so no host-to-device copy is needed either
-  int* counter = reinterpret_cast<int*>(b + kOffCounter);
-  noalloc_describe<<<(int)((n_units + 127) / 128), 128, 0, s>>>(blk, bd, counter, units, tiles,
-                                                                ranges, (int)n_units, (int)tiles_x,
-                                                                (int)tiles_y, (int)rpu);
+  g.tiles_x = (int)tiles_x;
+  g.tiles_y = (int)tiles_y;
+  g.slabs = (int)slabs;
+  g.runs = (int)pieces(std::min<int64_t>(I0, kTileX) * std::min<int64_t>(I1, kTileY) * pieces(I2, slabs), kAlgebraThreads);
 
   DerivArgs da;
   AlgebraArgs aa;
@@ -215,19 +219,8 @@ extern "C" int b200bssn_rhs_noalloc(double* const* rhs_dev, const double* const*
     aa.u[v] = u_dev[v];
     aa.rhs[v] = rhs_dev[v];
   }
-  da.blocks = aa.blocks = bd;
-  da.units = aa.units = units;
-  da.tiles = tiles;
-  aa.ranges = ranges;
-  da.dscr = b + kOffDeriv;
-  aa.dscr = b + kOffDeriv;
-  da.koscr = b + kOffKo;
-  aa.koscr = da.koscr;
-  da.cap = aa.cap = (int32_t)kNoallocMaxPoints;
-  da.tile_base = 0;
-  da.tile_count = (int32_t)(n_units * tiles_x * tiles_y);
-  da.counter = counter;
-  aa.range_base = 0;
+  da.scr = setup.addr;
+  aa.scr = setup.addr;
   aa.prm64 = {(double)prm->lambda[0], (double)prm->lambda[1], (double)prm->lambda[2],
               (double)prm->lambda[3], prm->lambda_f[0], prm->lambda_f[1]};
   aa.prm32 = {(float)prm->lambda[0], (float)prm->lambda[1], (float)prm->lambda[2],
@@ -237,17 +230,21 @@ extern "C" int b200bssn_rhs_noalloc(double* const* rhs_dev, const double* const*
   aa.eta_damping_exp = prm->eta_damping_exp;
   aa.ko_sigma = prm->ko_sigma;
 
-  const int64_t items = n_units * tiles_x * tiles_y * kNumVars;
-  const int64_t gmax = prm->precision == B200BSSN_MIXED ? grid32 : grid64;
-  const dim3 g1((unsigned)(items < gmax ? items : gmax), 1);
-  const unsigned g2 = (unsigned)(n_units * rpu);  // runs past a unit's end have count 0
-  if (prm->precision == B200BSSN_MIXED) {
-    bssn_derivs_kernel<float><<<g1, kDerivThreads, kDerivSmemBytes, s>>>(da);
-    bssn_algebra_kernel<float, float><<<g2, kAlgebraThreads, 0, s>>>(aa);
-  } else {
-    bssn_derivs_kernel<double><<<g1, kDerivThreads, kDerivSmemBytes, s>>>(da);
-    bssn_algebra_kernel<double, double><<<g2, kAlgebraThreads, 0, s>>>(aa);
+  const bool mixed = prm->precision == B200BSSN_MIXED;
+  const bool closure = blk.bflag != 0;
+  for (int k = 1; k >= 0; --k) {
+    void* arg[] = {&da, &g};
+    const void* fn = mixed ? derivs_kernel<float>(k == 1, closure) : derivs_kernel<double>(k == 1, closure);
+    if (launch_deriv(fn, (int)n_tiles * kKindVars[k], arg, k == 0, s) != cudaSuccess) {
+      cudaGetLastError();
+      return B200BSSN_ERR_CUDA;
+    }
   }
+  const unsigned grid = (unsigned)(n_tiles * g.runs);
+  if (mixed)
+    noalloc_algebra<float><<<grid, kAlgebraThreads, 0, s>>>(aa, g);
+  else
+    noalloc_algebra<double><<<grid, kAlgebraThreads, 0, s>>>(aa, g);
   if (cudaGetLastError() != cudaSuccess) return B200BSSN_ERR_CUDA;
   return B200BSSN_OK;
 }

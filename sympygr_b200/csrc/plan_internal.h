@@ -17,8 +17,8 @@ struct ConstraintArgs;
 
 using b200bssn::BlockDev;
 using b200bssn::RangeDev;
+using b200bssn::SlabDev;
 using b200bssn::TileDev;
-using b200bssn::UnitDev;
 
 struct b200bssn_ctx {
   int device = 0;
@@ -43,6 +43,7 @@ struct b200bssn_ctx {
 
 struct ChunkRec {
   int32_t tile_begin, tile_count;
+  int32_t list[3];  // how many of them take which closure rows (TileClosure): `order` holds them so
   int32_t range_begin, range_count;
   int64_t points;
 };
@@ -52,26 +53,29 @@ struct b200bssn_plan {
   uint32_t precision = 0;
   bool advective = false;  // upwind mode: 72 more scratch slots (advective derivatives)
   std::vector<BlockDev> blocks;
-  std::vector<UnitDev> units;
+  std::vector<SlabDev> slabs;
   std::vector<TileDev> tiles;
+  std::vector<int32_t> order;  // per chunk its tiles in the order the derivative kernels take them
   std::vector<RangeDev> ranges;
   std::vector<ChunkRec> chunks;
   uint64_t points = 0;
-  int64_t cap = 0;
+  int64_t cap = 0;  // scratch points of a buffer
   uint64_t span_lo = 0, span_hi = 0;  // element range touched in the variable arrays
   // device
-  void* desc = nullptr;  // blocks | units | tiles | ranges
+  void* desc = nullptr;  // blocks | slabs | tiles | order | ranges
   BlockDev* d_blocks = nullptr;
-  UnitDev* d_units = nullptr;
+  SlabDev* d_slabs = nullptr;
   TileDev* d_tiles = nullptr;
+  int32_t* d_order = nullptr;
   RangeDev* d_ranges = nullptr;
-  // derivative scratch: two buffers when the plan has more than one chunk, so the
-  // derivative kernel of chunk c+1 can run while the algebra kernel of chunk c reads
-  void* dscr[2] = {nullptr, nullptr};
-  void* koscr[2] = {nullptr, nullptr};  // KO sums, stored like the slots (double or float)
+  // derivative scratch (num_slots slots per scratch point, double or float): two buffers when
+  // the plan has more than one chunk, so the derivative kernels of chunk c+1 can run while the
+  // algebra kernel of chunk c reads
+  void* scr[2] = {nullptr, nullptr};
+  uint8_t* up[2] = {nullptr, nullptr};  // upwind mode: the shift's signs per scratch point
   std::vector<cudaEvent_t> ev_deriv, ev_alg;  // per chunk: derivative / algebra done
   cudaEvent_t ev_fork = nullptr;
-  int* d_counters = nullptr;  // per chunk: work counter of the derivative kernel
+  int* d_counters = nullptr;  // work counters of an evaluation
   unsigned long long* d_guard = nullptr;  // finiteness check result (allocated on first use)
   // pipelined host path: element ranges [part[c], part[c+1]) partition the span, one
   // per chunk, when chunks hold whole blocks in increasing offset order
@@ -79,11 +83,10 @@ struct b200bssn_plan {
   std::vector<uint64_t> part;
   std::vector<std::vector<int32_t>> chunk_blocks;  // per chunk: its blocks (host pipeline)
   std::vector<cudaEvent_t> ev_in;  // per chunk: upload done
-  int tile_y = b200bssn::kTileY;      // tile height of the derivative kernels (4, 8 or 16)
-  int deriv_regs = 0;                 // register split variant of the derivative kernels
-  const void* kind_fn[2] = {nullptr, nullptr};  // the derivative kind kernels (without / with DD)
-  int deriv_threads = 128;            // threads per derivative CTA
-  int deriv_grid[2] = {0, 0};  // resident CTAs of the two persistent derivative kernels
+  // the derivative kernels [kind: without / with second derivatives][TileClosure]
+  // and their resident CTAs
+  const void* kind_fn[2][3] = {};
+  int deriv_grid[2][3] = {};
   int alg_grid = 0;           // resident CTAs of the persistent staged algebra kernel (MIXED)
   // one-pass path (MIXED, centred advection): tile-slabs in launch order, the
   // per-evaluation sync words and the scratch ring
@@ -94,8 +97,7 @@ struct b200bssn_plan {
   b200bssn::FusedTileDev* d_ftiles = nullptr;
   int* d_fsync = nullptr;
   size_t fsync_words = 0;
-  void* fring_d = nullptr;  // nring * kFusedSlotPts points x 138 slots (float)
-  void* fring_k = nullptr;  // nring * kFusedSlotPts points x 24 KO sums (float)
+  void* fring = nullptr;  // nring * kFusedSlotPts points, all slots (float)
   // host-batch staging (allocated on first host call)
   double* st_u = nullptr;
   double* st_rhs = nullptr;
