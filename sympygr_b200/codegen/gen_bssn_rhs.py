@@ -399,10 +399,14 @@ def main_split(args):
         at = [i for i, st in enumerate(stages) if st[0] == "R"][0]
         defs = stages[at][1]
         stages = stages[:at] + [("R_a", defs[:3]), ("R_b", defs[3:])] + stages[at + 1:]
+    # the complete Christoffels of part 0 only after the Ricci tensor, which does not use them:
+    # eighteen values less to hold through the stage with the most temporaries
+    late = [st for st in stages if st[0] == "C3"]
+    part0_stages = [st for st in stages[:-1] if st[0] != "C3"] + late + stages[-1:]
     parts = [SPLIT_PART0, [n for n in src.RHS_NAMES if n not in SPLIT_PART0]]
     texts, stats = [], {}
     for p, outs in enumerate(parts):
-        body, nops, ntmp = emit_staged(prune_stages(stages, set(outs)), CudaPrinter(), slots)
+        body, nops, ntmp = emit_staged(prune_stages(part0_stages if p == 0 else stages, set(outs)), CudaPrinter(), slots)
         stats["nops%d" % p], stats["ntmp%d" % p] = nops, ntmp
         texts.append(
             "template <>\nstruct RhsAlgebraPart<%d> {\n"

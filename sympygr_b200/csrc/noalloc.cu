@@ -151,10 +151,15 @@ noalloc_algebra(const __grid_constant__ AlgebraArgs a, const __grid_constant__ N
   const uint32_t td = (uint32_t)nblk * NS * 32 * sizeof(ST);
   for (uint32_t off = 4096u * threadIdx.x; off < td; off += 4096u * kAlgebraThreads)
     prefetch_l2_bulk(pd + off, min(4096u, td - off));
-  if ((int)threadIdx.x >= count) return;
-  const int lp = start + threadIdx.x, r = lp / t.ex, z = r / t.ey;
-  const GlobalScratch<ST> src{static_cast<const ST*>(a.scr) + scr_index<NS>(0, t.sbase + lp)};
-  algebra_point_at<ST, RK_NONE>(a, g.block, 3 + t.i0 + (lp - r * t.ex), 3 + t.j0 + (r - z * t.ey), 3 + t.k0 + z, src);
+  const bool valid = (int)threadIdx.x < count;
+  const int lp = start + (valid ? threadIdx.x : 0), r = lp / t.ex, z = r / t.ey;
+  const int i = 3 + t.i0 + (lp - r * t.ex), j = 3 + t.j0 + (r - z * t.ey), k = 3 + t.k0 + z;
+  const ST* const scr = static_cast<const ST*>(a.scr);
+  const bool face = face_points<RK_NONE>(a, g.block, i, j, k, valid, [&](int l) {
+    return GlobalScratch<ST>{scr + scr_index<NS>(0, __shfl_sync(0xffffffffu, t.sbase + lp, l))};
+  });
+  if (valid && !face)
+    algebra_point_at<ST, RK_NONE>(a, g.block, i, j, k, GlobalScratch<ST>{scr + scr_index<NS>(0, t.sbase + lp)});
 }
 
 }  // namespace

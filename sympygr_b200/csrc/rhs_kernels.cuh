@@ -94,17 +94,26 @@ struct PointIn {
 // parameter so each instantiation is straight-line code: a run-time branch per
 // output splits the generated algebra into basic blocks the scheduler cannot
 // interleave across (measured: the algebra kernel ran 2x slower).
+struct StageIn { double base, acc; };  // what the update reads: u^n and the accumulator
 template <int MODE>
-__device__ __forceinline__ void store_rhs(const AlgebraArgs& a, int v, int64_t pp, double k) {
+__device__ __forceinline__ StageIn stage_in(const AlgebraArgs& a, int v, int64_t pp) {
+  StageIn in{};
+  if constexpr (MODE == RK_FIRST || MODE == RK_MIDDLE) in.base = __ldg(a.rk.base[v] + pp);
+  if constexpr (MODE == RK_LAST) in.base = a.rk.base[v][pp];
+  if constexpr (MODE == RK_MIDDLE || MODE == RK_LAST) in.acc = a.rk.acc[v][pp];
+  return in;
+}
+template <int MODE>
+__device__ __forceinline__ void store_rhs(const AlgebraArgs& a, int v, int64_t pp, double k, const StageIn& in) {
   const RkStage& rk = a.rk;
   if constexpr (MODE == RK_LAST) {
-    rk.base[v][pp] = rk.base[v][pp] + rk.acc[v][pp] + rk.w * k;
+    rk.base[v][pp] = in.base + in.acc + rk.w * k;
   } else if constexpr (MODE == RK_FIRST) {
     rk.acc[v][pp] = rk.w * k;
-    rk.next[v][pp] = __ldg(rk.base[v] + pp) + rk.c * k;
+    rk.next[v][pp] = in.base + rk.c * k;
   } else if constexpr (MODE == RK_MIDDLE) {
-    rk.acc[v][pp] = rk.acc[v][pp] + rk.w * k;
-    rk.next[v][pp] = __ldg(rk.base[v] + pp) + rk.c * k;
+    rk.acc[v][pp] = in.acc + rk.w * k;
+    rk.next[v][pp] = in.base + rk.c * k;
   } else {
     a.rhs[v][pp] = k;
   }
@@ -118,7 +127,7 @@ struct PointSink {
   template <typename RT>
   __device__ __forceinline__ void put(int v, RT val) {
     // rhs += sigma * (ko_x + ko_y + ko_z), rounded as rhs.cpp:332-369 rounds it
-    store_rhs<MODE>(*a, v, pp, __dadd_rn((double)val, __dmul_rn(a->ko_sigma, src.kov(v))));
+    store_rhs<MODE>(*a, v, pp, __dadd_rn((double)val, __dmul_rn(a->ko_sigma, src.kov(v))), stage_in<MODE>(*a, v, pp));
   }
 };
 
@@ -126,44 +135,99 @@ __device__ __forceinline__ void prefetch_l2_bulk(const void* p, uint32_t bytes) 
   asm volatile("cp.async.bulk.prefetch.L2.global [%0], %1;" ::"l"(p), "r"(bytes) : "memory");
 }
 
-// FP64 algebra as the two-part split of bssn_rhs_algebra_split.cuh
-constexpr bool kSplitAlgebra64 = true;
+__device__ __forceinline__ bool on_flagged_face(const BlockDev& B, int i, int j, int k) {
+  const uint32_t bf = B.bflag;
+  return ((bf & 1u) && i == 3) || ((bf & 2u) && i == B.sz[0] - 4) || ((bf & 4u) && j == 3) ||
+         ((bf & 8u) && j == B.sz[1] - 4) || ((bf & 16u) && k == 3) || ((bf & 32u) && k == B.sz[2] - 4);
+}
 
-// The right-hand side of interior point (i, j, k) (padded coordinates) of block B,
-// inputs through `src`.
-template <typename RT, int MODE, class Src, bool ADV = false>
-__device__ __forceinline__ void algebra_point_at(const AlgebraArgs& a, const BlockDev& B, int i, int j,
-                                                 int k, const Src& src) {
-  const int nx = B.sz[0], ny = B.sz[1];
-  const int64_t pp = B.offset + i + (int64_t)nx * (j + (int64_t)ny * k);
-  // coordinates as bssnrhs forms them (pmin + i*h, two roundings, rhs.cpp:207-213)
+// coordinates as bssnrhs forms them (pmin + i*h, two roundings, rhs.cpp:207-213)
+struct PointPos {
+  double x, y, z, r2;
+};
+__device__ __forceinline__ PointPos point_pos(const BlockDev& B, int i, int j, int k) {
   const double x = __dadd_rn(B.pmin[0], __dmul_rn((double)i, B.h[0]));
   const double y = __dadd_rn(B.pmin[1], __dmul_rn((double)j, B.h[1]));
   const double z = __dadd_rn(B.pmin[2], __dmul_rn((double)k, B.h[2]));
-  const double r2 = __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z));
-  const uint32_t bf = B.bflag;
-  const bool on_face = ((bf & 1u) && i == 3) || ((bf & 2u) && i == nx - 4) ||
-                       ((bf & 4u) && j == 3) || ((bf & 8u) && j == ny - 4) ||
-                       ((bf & 16u) && k == 3) || ((bf & 32u) && k == B.sz[2] - 4);
-  if (on_face) {
-    // bssn_bcs (rhs.cpp:833-977) replaces the algebra on face planes; KO is added
-    // afterwards (rhs.cpp:323-369).
-    const double inv_r = 1.0 / sqrt(r2);
-#pragma unroll 1
-    for (int v = 0; v < kNumVars; ++v) {
-      const double f = __ldg(a.u[v] + pp);
-      const double dxf = (double)src.dv(3 * v + 0);
-      const double dyf = (double)src.dv(3 * v + 1);
-      const double dzf = (double)src.dv(3 * v + 2);
-      double t = __dmul_rn(x, dxf);
-      t = __dadd_rn(t, __dmul_rn(y, dyf));
-      t = __dadd_rn(t, __dmul_rn(z, dzf));
-      t = __dadd_rn(t, __dmul_rn(bc_falloff(v), __dsub_rn(f, bc_asymptotic(v))));
-      const double val = __dmul_rn(-inv_r, t);
-      store_rhs<MODE>(a, v, pp, __dadd_rn(val, __dmul_rn(a.ko_sigma, src.kov(v))));
+  return {x, y, z, __dadd_rn(__dadd_rn(__dmul_rn(x, x), __dmul_rn(y, y)), __dmul_rn(z, z))};
+}
+
+// The face planes of a warp's points: bssn_bcs (rhs.cpp:833-977) replaces the algebra there,
+// KO is added afterwards (rhs.cpp:323-369).  The whole warp calls it, each lane with its own
+// point (`valid`: it has one); `at(l)` is the scratch of lane l's point.  Returns whether
+// the lane's point lies on a face, and so is done.
+// A row meets the two x faces with one point each, so nearly every warp of a flagged block has
+// one such lane, and its 24 variables one after another -- a load from L2 and a chain of
+// FP64 operations each -- took as long as the algebra of all the others.  The (face point,
+// variable) pairs are therefore shared out over the lanes, kFaceBatch loads in flight per lane.
+// Per evaluation of 64 blocks of 37^3 with all faces flagged (1.9 M points) the algebra took
+// 0.91 ms (MIXED) and 1.19 ms (FP64) with each lane looping over its own variables, 0.43 and
+// 0.69 ms without faces; so shared out 0.49 and 0.76 ms.
+constexpr int kFaceBatch = 4;
+template <int MODE, class At>
+__device__ __forceinline__ bool face_points(const AlgebraArgs& a, const BlockDev& B, int i, int j, int k, bool valid,
+                                            const At& at) {
+  if (B.bflag == 0) return false;
+  const bool mine = valid && on_flagged_face(B, i, j, k);
+  const uint32_t mask = __ballot_sync(0xffffffffu, mine);
+  if (mask == 0) return false;
+  const int lane = threadIdx.x & 31, n = __popc(mask);
+  // the lane of face point `lane`
+  int owner = 0;
+#pragma unroll
+  for (int step = 16; step > 0; step >>= 1)
+    if (__popc(mask & ((1u << (owner + step)) - 1u)) <= lane) owner += step;
+  const PointPos P = point_pos(B, i, j, k);
+  const double inv_r = mine ? 1.0 / sqrt(P.r2) : 0.0;
+  const int64_t pp = B.offset + i + (int64_t)B.sz[0] * (j + (int64_t)B.sz[1] * k);
+  const int dv = 32 / n, dq = 32 - dv * n;
+  int v = lane / n, q = lane - v * n;  // this lane's variable and face point
+  for (int pass = 0; pass < (kNumVars * n + 31) / 32; pass += kFaceBatch) {
+    int va[kFaceBatch], from[kFaceBatch];
+    int64_t pa[kFaceBatch];
+    double f[kFaceBatch], d[kFaceBatch][3], ko[kFaceBatch];
+    StageIn in[kFaceBatch];
+#pragma unroll
+    for (int b = 0; b < kFaceBatch; ++b) {
+      from[b] = __shfl_sync(0xffffffffu, owner, q);
+      pa[b] = __shfl_sync(0xffffffffu, pp, from[b]);
+      const auto src = at(from[b]);
+      va[b] = v;
+      if (v < kNumVars) {
+        f[b] = __ldg(a.u[v] + pa[b]);
+        in[b] = stage_in<MODE>(a, v, pa[b]);
+#pragma unroll
+        for (int x = 0; x < 3; ++x) d[b][x] = (double)src.dv(3 * v + x);
+        ko[b] = src.kov(v);
+      }
+      v += dv;
+      q += dq;
+      if (q >= n) q -= n, ++v;
     }
-    return;
+#pragma unroll
+    for (int b = 0; b < kFaceBatch; ++b) {
+      const double x = __shfl_sync(0xffffffffu, P.x, from[b]), y = __shfl_sync(0xffffffffu, P.y, from[b]);
+      const double z = __shfl_sync(0xffffffffu, P.z, from[b]), ir = __shfl_sync(0xffffffffu, inv_r, from[b]);
+      if (va[b] < kNumVars) {
+        double t = __dmul_rn(x, d[b][0]);
+        t = __dadd_rn(t, __dmul_rn(y, d[b][1]));
+        t = __dadd_rn(t, __dmul_rn(z, d[b][2]));
+        t = __dadd_rn(t, __dmul_rn(bc_falloff(va[b]), __dsub_rn(f[b], bc_asymptotic(va[b]))));
+        const double val = __dmul_rn(-ir, t);
+        store_rhs<MODE>(a, va[b], pa[b], __dadd_rn(val, __dmul_rn(a.ko_sigma, ko[b])), in[b]);
+      }
+    }
   }
+  return mine;
+}
+
+// The right-hand side of interior point (i, j, k) (padded coordinates) of block B, off its
+// flagged faces, inputs through `src`.
+template <typename RT, int MODE, class Src, bool ADV = false>
+__device__ __forceinline__ void algebra_point_at(const AlgebraArgs& a, const BlockDev& B, int i, int j,
+                                                 int k, const Src& src) {
+  const int64_t pp = B.offset + i + (int64_t)B.sz[0] * (j + (int64_t)B.sz[1] * k);
+  const double r2 = point_pos(B, i, j, k).r2;
   // eta damping, rhs.cpp:213-219
   const double r_coord = sqrt(r2);
   double eta = a.eta_const;
@@ -178,10 +242,14 @@ __device__ __forceinline__ void algebra_point_at(const AlgebraArgs& a, const Blo
     prm = &a.prm32;
   if constexpr (ADV) {
     bssn_rhs_algebra_adv<RT>(in, sink, *prm, (RT)eta);
-  } else if constexpr (sizeof(RT) == 8 && kSplitAlgebra64) {
+  } else if constexpr (sizeof(RT) == 8) {
     // FP64: the algebra in two parts (the six At_rhs with the Ricci tensor, then the
-    // rest), each with its own live set
+    // rest), each with its own live set: the opaque offset between them keeps the compiler from
+    // holding values of the first for the second.  At 255 registers what spills -- 72 bytes --
+    // counts: shared memory leaves little L1, and the same kernel with 340 bytes took 1.60
+    // instead of 1.36 ms on 16 blocks of 69^3
     RhsAlgebraPart<0>::run<RT>(in, sink, *prm, (RT)eta);
+    asm volatile("" : "+l"(in.pp));
     RhsAlgebraPart<1>::run<RT>(in, sink, *prm, (RT)eta);
   } else {
     bssn_rhs_algebra<RT>(in, sink, *prm, (RT)eta);
@@ -212,7 +280,10 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
   ST* sd = reinterpret_cast<ST*>(s_stage + warp * Cfg::kBytesPerWarp);
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(sd)) + 16u * (uint32_t)lane;
   const int nwarps = gridDim.x * Cfg::kWarps;
-  for (int task = blockIdx.x * Cfg::kWarps + warp; task < ntasks; task += nwarps) {
+  // Neighbouring tasks share state and scratch lines and go to one CTA; fewer tasks than warps
+  // are spread over the SMs first.
+  const int first = ntasks < nwarps ? warp * gridDim.x + blockIdx.x : blockIdx.x * Cfg::kWarps + warp;
+  for (int task = first; task < ntasks; task += nwarps) {
     const RangeDev rg = a.ranges[a.range_base + task / kRangeTasks];
     if ((task & (kRangeTasks - 1)) >= rg.count) continue;
     const SlabDev slab = a.slabs[rg.slab];
@@ -259,11 +330,9 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
     cp_async_commit();
     cp_async_wait<0>();
     __syncwarp();  // the copies of every lane are visible to the whole warp
-    if (p.valid) {
-      using Src = SharedScratch<ST, Cfg::kAll>;
-      const Src src{sd + lane, own};
-      algebra_point_at<RT, MODE, Src, ADV>(a, B, p.i, p.j, p.k, src);
-    }
+    using Src = SharedScratch<ST, Cfg::kAll>;
+    const bool face = face_points<MODE>(a, B, p.i, p.j, p.k, p.valid, [sd, own](int l) { return Src{sd + l, own}; });
+    if (p.valid && !face) algebra_point_at<RT, MODE, Src, ADV>(a, B, p.i, p.j, p.k, Src{sd + lane, own});
   }
 }
 
