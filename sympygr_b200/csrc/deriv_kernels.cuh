@@ -17,22 +17,27 @@
 //     D_z(D_y).  unroll_planes planes are processed per loop pass, so the register windows
 //     move once per pass.
 //
-// What bounds it: see plan_types.h for the stores.  With those filling whole sectors, the
-// kernel that this one replaced (one column per thread, CTAs of 4 warps, 8-byte copies, one
-// plane per barrier and pass) issued 94 / 136 instructions per point (without / with second
-// derivatives, MIXED) and kept the shared-memory data pipe 81 / 70 % busy; sharing the y
-// windows, 16-byte copies and the unrolled passes bring that to 60 / 100 instructions.
+// What bounds it: see plan_types.h for the stores.  The kernel that this one replaced (one
+// column per thread, CTAs of 4 warps, 8-byte copies, one plane per barrier and pass) kept the
+// shared-memory data pipe 81 / 70 % busy (without / with second derivatives) once its stores
+// filled whole sectors; sharing the y windows, 16-byte copies and the unrolled passes bring that
+// to 59 %, the issue slots to 65 / 60 % and DRAM to 52 / 44 % of its peak (64 blocks of 37^3,
+// MIXED): no single resource is full, and what is left is the latency of 16 / 12 warps per SM.
+// 16 blocks of 69^3 (4.0 M points): 0.83 ms (MIXED) and 1.14 ms (FP64), before 1.46 and 2.00 ms.
 //
 // Closure rows (within three points of a flagged face) reach no further than three points
-// beyond a tile or slab (cut_start), except that the D rows at the face itself reach four
-// planes along z: those are formed one plane later (low side) or earlier (high side), when
-// the window holds all their planes.  The item's code is instantiated without closure rows,
-// with those along z (a branch that all threads take together) and with all (TileClosure),
-// in kernels of their own: compiled into the common path the z branch alone cost it 18 %
-// (16 blocks of 69^3, MIXED: 1.01 against 0.86 ms).  The closure rows along x and y are spread
-// over all threads first: evaluated where they occur, by a few lanes of every warp, they took
-// tiles at such faces 3.5 times as long as others, shared out twice as long (16 blocks of 69^3
-// with all faces flagged, MIXED: 2.27 and 1.72 ms; 3.65 ms with one column per thread).
+// beyond a tile or slab (cut_start).  Along z the three rows of a face are formed together,
+// at the plane whose window holds the six that they read.  The item's code is instantiated
+// without closure rows, with those along z (a branch that all threads take together) and with
+// all (TileClosure), in kernels of their own: compiled into the common path the z branch alone
+// cost it 18 % (16 blocks of 69^3, MIXED: 1.01 against 0.86 ms).  One code runs for all six
+// rows, their weights in shared memory: a copy per row, inlined for each of a pass's planes
+// and columns, left the kernel waiting for instructions a fifth of its time.  The closure rows
+// along x and y are spread over all threads first: evaluated where they occur, by a few lanes
+// of every warp, they took tiles at such faces 3.5 times as long as others.  64 blocks of 37^3
+// with all faces flagged: 0.93 ms (MIXED) and 1.03 ms (FP64); with the z rows copied out and
+// every thread working out its closure points anew in each plane 1.10 and 1.25 ms; 0.46 and
+// 0.60 ms without faces.  16 blocks of 69^3: 1.39 and 1.62 ms, before 3.65 and 4.13 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -80,10 +85,16 @@ struct alignas(16) DerivSmem {
   double dx[DD ? kDxPlane : 1];
   LineScales sc[3];
 };
-// Closure values of a plane (d1, ko, d2), by row id: of the three columns next to a face
-// flagged along x, every staged row; of the three rows next to a face flagged along y.
+// Closure values of a plane: d1, ko, d2 of the columns next to faces flagged along x (staged
+// row by staged row, three columns a face), then of the rows next to faces flagged along y
+// (row by row); and where each one's points lie (closure_point).  Before them ko_x + ko_y of
+// the last kKoPlanes planes, which the closure rows along z take from here.
+constexpr int kKoPlanes = 8;
+constexpr int kClosurePoints = 2 * 3 * kPlaneRows + 2 * 3 * kTileX;
 struct ClosureValues {
-  double x[3][6][kPlaneRows], y[3][6][kTileX];
+  double ko[kKoPlanes][kTilePlane];
+  double v[3][kClosurePoints];
+  int32_t point[kClosurePoints];
 };
 struct ClosureRow;
 
@@ -101,98 +112,6 @@ __device__ __forceinline__ int z_case(int zo, int n, bool lo, bool hi) {
   if (lo && zo < 6) return zo - 3;
   return -1;
 }
-
-// The closure rows along z on a window q[0..8] holding planes zo-4 .. zo+4 of one column;
-// every index is compile-time, so the window stays in registers.  Same operations and
-// order as line_*.
-#define ZQ(k) ((double)q[(k)])
-template <typename T>
-__device__ __forceinline__ double zq_d1_closure(const T (&q)[9], int zc, const LineScales& c) {
-  double a;
-  switch (zc) {
-    case 0:  // zo=3: planes 3..7 -> q[4..8]
-      a = __dmul_rn(-25.0, ZQ(4)); a = mad_rn(a, 48.0, ZQ(5)); a = mad_rn(a, -36.0, ZQ(6));
-      a = mad_rn(a, 16.0, ZQ(7)); a = mad_rn(a, -3.0, ZQ(8));
-      break;
-    case 1:  // zo=4: planes 3..7 -> q[3..7]
-      a = __dmul_rn(-3.0, ZQ(3)); a = mad_rn(a, -10.0, ZQ(4)); a = mad_rn(a, 18.0, ZQ(5));
-      a = mad_rn(a, -6.0, ZQ(6)); a = mad_rn(a, 1.0, ZQ(7));
-      break;
-    case 2:  // zo=5: planes 3,4,6,7 -> q[2,3,5,6]
-    case 3:  // zo=n-6: planes n-8,n-7,n-5,n-4 -> q[2,3,5,6]
-      a = __dmul_rn(1.0, ZQ(2)); a = mad_rn(a, -8.0, ZQ(3)); a = mad_rn(a, 8.0, ZQ(5));
-      a = mad_rn(a, -1.0, ZQ(6));
-      break;
-    case 4:  // zo=n-5: planes n-8..n-4 -> q[1..5]
-      a = __dmul_rn(-1.0, ZQ(1)); a = mad_rn(a, 6.0, ZQ(2)); a = mad_rn(a, -18.0, ZQ(3));
-      a = mad_rn(a, 10.0, ZQ(4)); a = mad_rn(a, 3.0, ZQ(5));
-      break;
-    default:  // 5: zo=n-4: planes n-8..n-4 -> q[0..4]
-      a = __dmul_rn(3.0, ZQ(0)); a = mad_rn(a, -16.0, ZQ(1)); a = mad_rn(a, 36.0, ZQ(2));
-      a = mad_rn(a, -48.0, ZQ(3)); a = mad_rn(a, 25.0, ZQ(4));
-      break;
-  }
-  return __dmul_rn(a, c.d1_b);
-}
-
-template <typename T>
-__device__ __forceinline__ double zq_d2_closure(const T (&q)[9], int zc, const LineScales& c) {
-  double a;
-  switch (zc) {
-    case 0:
-      a = __dmul_rn(35.0, ZQ(4)); a = mad_rn(a, -104.0, ZQ(5)); a = mad_rn(a, 114.0, ZQ(6));
-      a = mad_rn(a, -56.0, ZQ(7)); a = mad_rn(a, 11.0, ZQ(8));
-      break;
-    case 1:
-      a = __dmul_rn(11.0, ZQ(3)); a = mad_rn(a, -20.0, ZQ(4)); a = mad_rn(a, 6.0, ZQ(5));
-      a = mad_rn(a, 4.0, ZQ(6)); a = mad_rn(a, -1.0, ZQ(7));
-      break;
-    case 2:
-    case 3:
-      a = __dmul_rn(-1.0, ZQ(2)); a = mad_rn(a, 16.0, ZQ(3)); a = mad_rn(a, -30.0, ZQ(4));
-      a = mad_rn(a, 16.0, ZQ(5)); a = mad_rn(a, -1.0, ZQ(6));
-      break;
-    case 4:
-      a = __dmul_rn(-1.0, ZQ(1)); a = mad_rn(a, 4.0, ZQ(2)); a = mad_rn(a, 6.0, ZQ(3));
-      a = mad_rn(a, -20.0, ZQ(4)); a = mad_rn(a, 11.0, ZQ(5));
-      break;
-    default:
-      a = __dmul_rn(11.0, ZQ(0)); a = mad_rn(a, -56.0, ZQ(1)); a = mad_rn(a, 114.0, ZQ(2));
-      a = mad_rn(a, -104.0, ZQ(3)); a = mad_rn(a, 35.0, ZQ(4));
-      break;
-  }
-  return __dmul_rn(a, c.d2_b);
-}
-
-template <typename T>
-__device__ __forceinline__ double zq_ko_closure(const T (&q)[9], int zc, const LineScales& c) {
-  double a;
-  switch (zc) {
-    case 0:  // (u6 - 3u5 + 3u4 - u3)/s3, planes 3..6 -> q[4..7]
-      a = ZQ(7); a = mad_rn(a, -3.0, ZQ(6)); a = mad_rn(a, 3.0, ZQ(5)); a = __dsub_rn(a, ZQ(4));
-      return __ddiv_rn(a, c.ko_s3);
-    case 1:  // planes 3..7 -> q[3..7]
-      a = ZQ(7); a = mad_rn(a, -6.0, ZQ(6)); a = mad_rn(a, 12.0, ZQ(5)); a = mad_rn(a, -10.0, ZQ(4));
-      a = mad_rn(a, 3.0, ZQ(3));
-      return __ddiv_rn(a, c.ko_s2);
-    case 2:  // planes 3..8 -> q[2..7]
-      a = ZQ(7); a = mad_rn(a, -6.0, ZQ(6)); a = mad_rn(a, 15.0, ZQ(5)); a = mad_rn(a, -19.0, ZQ(4));
-      a = mad_rn(a, 12.0, ZQ(3)); a = mad_rn(a, -3.0, ZQ(2));
-      return __ddiv_rn(a, c.ko_s1);
-    case 3:  // zo=n-6: planes n-9..n-4 -> q[1..6]
-      a = ZQ(1); a = mad_rn(a, -6.0, ZQ(2)); a = mad_rn(a, 15.0, ZQ(3)); a = mad_rn(a, -19.0, ZQ(4));
-      a = mad_rn(a, 12.0, ZQ(5)); a = mad_rn(a, -3.0, ZQ(6));
-      return __ddiv_rn(a, c.ko_s1);
-    case 4:  // zo=n-5: planes n-8..n-4 -> q[1..5]
-      a = ZQ(1); a = mad_rn(a, -6.0, ZQ(2)); a = mad_rn(a, 12.0, ZQ(3)); a = mad_rn(a, -10.0, ZQ(4));
-      a = mad_rn(a, 3.0, ZQ(5));
-      return __ddiv_rn(a, c.ko_s2);
-    default:  // 5: zo=n-4: planes n-7..n-4 -> q[1..4]
-      a = ZQ(1); a = mad_rn(a, -3.0, ZQ(2)); a = mad_rn(a, 3.0, ZQ(3)); a = __dsub_rn(a, ZQ(4));
-      return __ddiv_rn(a, c.ko_s3);
-  }
-}
-#undef ZQ
 
 // Centred-row arithmetic of the derivative kernel, by precision mode.
 //
@@ -312,7 +231,7 @@ struct RowsFor { using type = ExactRows; };
 template <>
 struct RowsFor<float> { using type = SplitRows; };
 
-// The closure rows of a line, for the points next to a flagged face in x or y.  Row id: 0..2
+// The closure rows of a line, for the points next to a flagged face.  Row id: 0..2
 // the points 3, 4, 5 at a low face, 3..5 the points n-6, n-5, n-4 at a high one (closure_id).
 // A row reads the values m[k], k points from the face point inwards.  d1 and d2 sum five of
 // them in ascending index order, with the row's weights; ko sums from the far point inwards,
@@ -382,6 +301,13 @@ struct ScratchMap {
 // 0.770, 4 planes 0.675 / 0.903: the longer pass spills).
 __host__ __device__ constexpr int unroll_planes(bool dd, bool cl, bool adv) { return dd || cl || adv ? 2 : 4; }
 
+// Where the points of a closure row lie in a staged plane: the offset of the face point, the
+// parity of its staged row, whether the row runs along y, and the row id.
+__device__ __forceinline__ int closure_point(int offset, int row, bool along_y, int id) {
+  return offset | (row & 1) << 9 | (int)along_y << 10 | id << 11;
+}
+static_assert(kPlane <= 512, "closure_point holds nine bits of offset");
+
 // Barrier over the kItemThreads threads of an item; `id` names it where a CTA runs several.
 __device__ __forceinline__ void item_sync(int id) {
   asm volatile("bar.sync %0, %1;" ::"r"(id), "n"(kItemThreads) : "memory");
@@ -416,10 +342,30 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
   int idy[R];
 #pragma unroll
   for (int r = 0; r < R; ++r) idy[r] = closure_id(gj0 + r, ny, loy, hiy);
+  // Closure points along x and y (ClosureValues): per = those of a face along x -- all staged
+  // rows with second derivatives, whose D_y(D_x) reads them, else the tile's own --, npx of both.
+  constexpr int kRow0 = DD ? 0 : kHalo;
   const bool flx = lox && i0 == 3, fhx = hix && i0 + ex == nx - 3, fly = loy && j0 == 3, fhy = hiy && j0 + ey == ny - 3;
   const uint32_t plane_elems = (uint32_t)nx * (uint32_t)ny;
   const int np = ez + 2 * kHalo;  // planes streamed: k0 - 3 .. k0 + ez + 2, all inside the block
   const int rows = ey + 2 * kHalo;
+  const int per = 3 * (DD ? rows : ey), npx = per * ((int)flx + (int)fhx), npc = npx + 3 * kTileX * ((int)fly + (int)fhy);
+  // this thread's values: along x of staged row w at fx + 3 w, along y of its row r at fy[r]
+  int fx = 0, fy[R] = {};
+  if constexpr (CL) {
+    fx = (idx >= 3 ? idx - 3 + (flx ? per : 0) : idx) - 3 * kRow0;
+#pragma unroll
+    for (int r = 0; r < R; ++r)
+      fy[r] = npx + (idy[r] >= 3 ? kTileX * (idy[r] - 3) + (fly ? 3 * kTileX : 0) : kTileX * idy[r]) + tx;
+    for (int e = tid; e < npc; e += kItemThreads) {
+      const bool along_y = e >= npx, first = along_y ? fly : flx;
+      const int each = along_y ? 3 * kTileX : per, f = along_y ? e - npx : e;
+      const bool hi = !first || f >= each;
+      const int g = first && hi ? f - each : f, k = along_y ? g / kTileX : g % 3;
+      const int row = along_y ? (hi ? ey - 1 : 0) + kHalo : kRow0 + g / 3, x = along_y ? g % kTileX : (hi ? ex - 1 : 0);
+      fix->point[e] = closure_point(row * kPlaneW + x + kHalo, row, along_y, hi ? k + 3 : k);
+    }
+  }
 
   // Copies: a plane is 14 rows of 12 sixteen-byte pieces, piece e (row e / 12) by thread
   // e % 64.  A row's pieces start at the 16-byte boundary at or before its first element.
@@ -484,7 +430,7 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
   const LineScales& cy = S.sc[1];
   const LineScales& cz = S.sc[2];
 
-  double U[R][6 + B], X[DD ? R : 1][6 + B], Y[DD ? R : 1][6 + B], K[R][NK + B];
+  double U[R][6 + B], X[DD ? R : 1][6 + B], Y[DD ? R : 1][6 + B], K[R][NK + B];  // (K: without closure rows along z)
 #pragma unroll
   for (int r = 0; r < R; ++r) {
 #pragma unroll
@@ -528,40 +474,22 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
           for (int r = 0; r < R; ++r) up_bits[r] = (up_bits[r] << 8) | (out ? up_next[r] : 0u);
           if (out) load_up(o + 1);
         }
-        if constexpr (CL) {
-          // the closure points of the plane: three columns of `rows` at each face along x, then
-          // three rows of 16 at each along y
-          const int per = 3 * rows, npx = per * ((int)flx + (int)fhx), npy = 3 * kTileX * ((int)fly + (int)fhy);
-          for (int e = tid; e < npx + npy; e += kItemThreads) {
+        if (CL && (DD || out)) {
+          for (int e = tid; e < npc; e += kItemThreads) {
+            const int pt = fix->point[e], id = pt >> 11;
+            const bool along_y = pt >> 10 & 1;
+            const uint32_t nxo = (uint32_t)nx & 1u, even = sh ^ (nxo & (uint32_t)(pt >> 9)), odd = even ^ (along_y ? nxo : 0u);
+            const int step = (along_y ? kPlaneW : 1) * (id >= 3 ? -1 : 1);
+            const double* const q = S.plane[0] + slot * kPlane + (pt & 511);
             double m[6];
-            int id;
-            const bool alongx = e < npx;
-            double* to;
-            if (alongx) {
-              const bool hi = !flx || e >= per;
-              const int f = e - (flx && hi ? per : 0), row = f / 3;
-              id = f - 3 * row + (hi ? 3 : 0);
-              const uint32_t shr = (sh + ((uint32_t)nx & (uint32_t)row)) & 1u;
-              const double* q = S.plane[0] + slot * kPlane + row * kPlaneW + (hi ? ex - 1 : 0) + kHalo + shr;
 #pragma unroll
-              for (int k = 0; k < 6; ++k) m[k] = q[hi ? -k : k];
-              to = &fix->x[0][id][row];
-            } else {
-              const bool hi = !fly || e - npx >= 3 * kTileX;
-              const int f = e - npx - (fly && hi ? 3 * kTileX : 0), x = f % kTileX, row = (hi ? ey - 1 : 0) + kHalo;
-              id = f / kTileX + (hi ? 3 : 0);
-#pragma unroll
-              for (int k = 0; k < 6; ++k) {
-                const int w = hi ? row - k : row + k;
-                m[k] = S.plane[0][slot * kPlane + w * kPlaneW + x + kHalo + ((sh + ((uint32_t)nx & (uint32_t)w)) & 1u)];
-              }
-              to = &fix->y[0][id][x];
+            for (int k = 0; k < 6; ++k) m[k] = q[k * step + (int)((k & 1) ? odd : even)];
+            const LineScales& sc = along_y ? cy : cx;
+            fix->v[0][e] = closure_d1(m, id, closure[id], sc);
+            if (out) {
+              fix->v[1][e] = closure_ko(m, id, closure[id], sc);
+              if (DD) fix->v[2][e] = closure_d2(m, id, closure[id], sc);
             }
-            const LineScales& sc = alongx ? cx : cy;
-            const int step = alongx ? 6 * kPlaneRows : 6 * kTileX;
-            to[0] = closure_d1(m, id, closure[id], sc);
-            to[step] = closure_ko(m, id, closure[id], sc);
-            if (DD) to[2 * step] = closure_d2(m, id, closure[id], sc);
           }
           item_sync(barrier);
         }
@@ -588,16 +516,20 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
               dyy = (ST)Rows::d2(wy, 3, cy);
             }
             if (CL && idx >= 0) {
-              dx = fix->x[0][idx][ty0 + r + kHalo];
-              kx = fix->x[1][idx][ty0 + r + kHalo];
-              if (DD) dxx = (ST)fix->x[2][idx][ty0 + r + kHalo];
+              const int e = fx + 3 * (ty0 + r + kHalo);
+              dx = fix->v[0][e];
+              kx = fix->v[1][e];
+              if (DD) dxx = (ST)fix->v[2][e];
             }
             if (CL && idy[r] >= 0) {
-              dy = fix->y[0][idy[r]][tx];
-              ky = fix->y[1][idy[r]][tx];
-              if (DD) dyy = (ST)fix->y[2][idy[r]][tx];
+              dy = fix->v[0][fy[r]];
+              ky = fix->v[1][fy[r]];
+              if (DD) dyy = (ST)fix->v[2][fy[r]];
             }
-            K[r][NK + p] = __dadd_rn(kx, ky);
+            if (CLZ)
+              fix->ko[o & (kKoPlanes - 1)][tid + kItemThreads * r] = __dadd_rn(kx, ky);
+            else
+              K[r][NK + p] = __dadd_rn(kx, ky);
             if (DD) {
               X[r][6 + p] = dx;
               Y[r][6 + p] = dy;
@@ -634,7 +566,7 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
 #pragma unroll
                 for (int m = 0; m < 7; ++m) w[m] = px[m - 3];
                 double dx = Rows::d1_field(w, 3, cx);
-                if (CL && idx >= 0) dx = fix->x[0][idx][row];
+                if (CL && idx >= 0) dx = fix->v[0][fx + 3 * row];
                 S.dx[row * kTileX + tx] = dx;
               }
             }
@@ -669,7 +601,8 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
               // rhs.cpp:332-369 sums (ko_x + ko_y) + ko_z; summed in FP64, stored like the
               // slots (FP32 in MIXED: the term enters the output scaled by sigma)
               const ST dz = (ST)Rows::d1(U[r], 3 + p, cz);
-              const ST ks = (ST)__dadd_rn(K[r][NK + p - 3], Rows::ko(U[r], 3 + p, cz));
+              const double kxy = CLZ ? fix->ko[oz & (kKoPlanes - 1)][tid + kItemThreads * r] : K[r][NK + p - 3];
+              const ST ks = (ST)__dadd_rn(kxy, Rows::ko(U[r], 3 + p, cz));
               ST dzz = ST(0), dxz = ST(0), dyz = ST(0);
               if (DD) {
                 dzz = (ST)Rows::d2(U[r], 3 + p, cz);
@@ -687,38 +620,39 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
                 }
               }
             }
-          } else {
+          } else if (zc == 2 || zc == 3) {
+            // The three closure rows of a face, with the one farthest from it: the window then
+            // holds the six planes that they read, m[k] the one k from the face plane.
+            const bool hi = zc == 3;
+            const int o0 = hi ? oz : oz - 2, id0 = hi ? 3 : 0;
 #pragma unroll
             for (int r = 0; r < R; ++r) {
-              // w[k]: plane k - 4 from the output, whose plane has window index 4 - shift
-              auto window = [&](const double (&q)[6 + B], int shift, double (&w)[9]) {
+              auto inwards = [&](const double (&w)[6 + B], double (&m)[6]) {
 #pragma unroll
-                for (int k = 0; k < 9; ++k) {
-                  const bool in = k - shift >= 0 && k - shift < 7;
-                  w[k] = in ? q[in ? k - shift + p : 0] : 0.0;
-                }
-              };
-              // D rows 0 and 5 (the planes on the faces) are formed with rows 1 and 4, one
-              // plane later and earlier, when the window holds the planes they reach
-              auto emit = [&](int zcase, int shift, int co) {
-                double w[9];
-                window(U[r], shift, w);
-                sd_first[co + 2 * 32] = (ST)zq_d1_closure(w, zcase, cz);
-                if (DD) {
-                  sd_second[co + 5 * 32] = (ST)zq_d2_closure(w, zcase, cz);
-                  window(X[DD ? r : 0], shift, w);
-                  sd_second[co + 2 * 32] = (ST)zq_d1_closure(w, zcase, cz);
-                  window(Y[DD ? r : 0], shift, w);
-                  sd_second[co + 4 * 32] = (ST)zq_d1_closure(w, zcase, cz);
-                }
+                for (int k = 0; k < 6; ++k) m[k] = hi ? w[5 + p - k] : w[1 + p + k];
               };
               if (r < nr) {
-                double w[9];
-                window(U[r], 1, w);
-                sd_ko[at(r, oz)] = (ST)__dadd_rn(K[r][NK + p - 3], zq_ko_closure(w, zc, cz));
-                if (zc != 0 && zc != 5) emit(zc, 1, at(r, oz));
-                if (zc == 1) emit(0, 2, at(r, oz - 1));
-                if (zc == 4) emit(5, 0, at(r, oz + 1));
+                double m[6];
+                inwards(U[r], m);
+#pragma unroll 1
+                for (int k = 0; k < 3; ++k) {
+                  const int id = id0 + k, c = at(r, o0 + k);
+                  const double kxy = fix->ko[(o0 + k) & (kKoPlanes - 1)][tid + kItemThreads * r];
+                  sd_first[c + 2 * 32] = (ST)closure_d1(m, id, closure[id], cz);
+                  sd_ko[c] = (ST)__dadd_rn(kxy, closure_ko(m, id, closure[id], cz));
+                  if (DD) sd_second[c + 5 * 32] = (ST)closure_d2(m, id, closure[id], cz);
+                }
+                if constexpr (DD) {
+                  double mx[6], my[6];
+                  inwards(X[r], mx);
+                  inwards(Y[r], my);
+#pragma unroll 1
+                  for (int k = 0; k < 3; ++k) {
+                    const int id = id0 + k, c = at(r, o0 + k);
+                    sd_second[c + 2 * 32] = (ST)closure_d1(mx, id, closure[id], cz);
+                    sd_second[c + 4 * 32] = (ST)closure_d1(my, id, closure[id], cz);
+                  }
+                }
               }
             }
           }
@@ -801,13 +735,13 @@ template <typename ST, bool DD, bool ADV, int CLOSURE>
 __global__ void __launch_bounds__(kItemThreads, kind_ctas_per_sm(DD, ADV, CLOSURE))
 bssn_derivs_kind_kernel(const __grid_constant__ DerivArgs a) {
   constexpr int NV = kKindVars[DD];
-  constexpr bool CL = CLOSURE == kClosureXY;
+  constexpr bool CL = CLOSURE == kClosureXY, CLZ = CLOSURE != kClosureNone;
   __shared__ DerivSmem<DD> S;
-  __shared__ ClosureRow s_closure[CL ? 6 : 1];
-  __shared__ __align__(8) unsigned char s_fix[CL ? sizeof(ClosureValues) : 8];
+  __shared__ ClosureRow s_closure[CLZ ? 6 : 1];
+  __shared__ __align__(8) unsigned char s_fix[CL ? sizeof(ClosureValues) : CLZ ? sizeof(ClosureValues::ko) : 8];
   __shared__ int s_item;
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  if (CL) load_closure_rows(s_closure);
+  if (CLZ) load_closure_rows(s_closure);
   for (;;) {
     __syncthreads();  // the previous item is finished with the shared memory
     if (threadIdx.x == 0) s_item = atomicAdd(a.counter, 1);

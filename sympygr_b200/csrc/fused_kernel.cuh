@@ -45,7 +45,9 @@
 namespace b200bssn {
 
 constexpr int kFusedThreads = 128;                              // 4 warps: one item or one algebra claim
-constexpr int kFusedMinBlocks = 3;                              // CTAs per SM (168 registers)
+// CTAs per SM: two, of 255 registers.  Three, of 168, spill 770 bytes of the algebra, and their
+// shared memory leaves little L1 to spill to (37^3, 64 blocks: 2.13 against 1.59 ms).
+constexpr int kFusedMinBlocks = 2;
 constexpr unsigned long long kFusedWaitNs = 2000000000ull;      // 2 s per wait, then an error
 constexpr size_t kFusedStageBytes = (size_t)kNumDerivs * kStageW * sizeof(float);  // per warp
 constexpr size_t kFusedSmemBytes = 4 * kFusedStageBytes;        // 70,656 B (derivative buffers alias it)
@@ -55,7 +57,7 @@ union DerivSmemAny {
   DerivSmem<true> dd;
   DerivSmem<false> nd;
 };
-static_assert(kFusedItemVars * sizeof(DerivSmemAny) <= kFusedSmemBytes, "the derivative items' buffers fit in the algebra staging area");
+static_assert(kFusedItemVars * (sizeof(DerivSmemAny) + sizeof(ClosureValues)) <= kFusedSmemBytes, "the derivative items' buffers fit in the algebra staging area");
 static_assert(kFusedSlotPts == kTilePlane * kFusedSlab, "a ring slot is a tile of the scratch layout");
 
 // Device words of one evaluation, zeroed before the launch:
@@ -177,7 +179,6 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
   extern __shared__ __align__(16) unsigned char smem[];
   __shared__ int s_role, s_idx, s_p0, s_np;
   __shared__ ClosureRow s_closure[6];
-  __shared__ ClosureValues s_fix[kFusedItemVars];
   load_closure_rows(s_closure);
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   int* const done = f.sync + 4;
@@ -186,6 +187,7 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
   int pending = -1;  // warp 0: the item this CTA holds
   const int half = threadIdx.x / kItemThreads;  // this thread's variable of an item
   DerivSmemAny& S = reinterpret_cast<DerivSmemAny*>(smem)[half];
+  ClosureValues* const s_fix = reinterpret_cast<ClosureValues*>(smem + kFusedItemVars * sizeof(DerivSmemAny));
 
   for (;;) {
     if (warp == 0) {
