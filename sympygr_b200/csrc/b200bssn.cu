@@ -117,31 +117,31 @@ void launch_algebra(const AlgebraArgs& aa, unsigned grid, int ntasks, cudaStream
   using Cfg = StageCfg<ST, ADV>;
   switch (aa.rk.mode) {
     case RK_FIRST:
-      bssn_algebra_staged_kernel<ST, RK_FIRST, ADV><<<grid, Cfg::kThreads, Cfg::kSmemBytes, s>>>(aa, ntasks);
+      bssn_algebra_staged_kernel<ST, RK_FIRST, ADV><<<grid, Cfg::kThreads, Cfg::smem_bytes(RK_FIRST), s>>>(aa, ntasks);
       break;
     case RK_MIDDLE:
-      bssn_algebra_staged_kernel<ST, RK_MIDDLE, ADV><<<grid, Cfg::kThreads, Cfg::kSmemBytes, s>>>(aa, ntasks);
+      bssn_algebra_staged_kernel<ST, RK_MIDDLE, ADV><<<grid, Cfg::kThreads, Cfg::smem_bytes(RK_MIDDLE), s>>>(aa, ntasks);
       break;
     case RK_LAST:
-      bssn_algebra_staged_kernel<ST, RK_LAST, ADV><<<grid, Cfg::kThreads, Cfg::kSmemBytes, s>>>(aa, ntasks);
+      bssn_algebra_staged_kernel<ST, RK_LAST, ADV><<<grid, Cfg::kThreads, Cfg::smem_bytes(RK_LAST), s>>>(aa, ntasks);
       break;
     default:
-      bssn_algebra_staged_kernel<ST, RK_NONE, ADV><<<grid, Cfg::kThreads, Cfg::kSmemBytes, s>>>(aa, ntasks);
+      bssn_algebra_staged_kernel<ST, RK_NONE, ADV><<<grid, Cfg::kThreads, Cfg::smem_bytes(RK_NONE), s>>>(aa, ntasks);
       break;
   }
 }
 
 template <typename ST, bool ADV>
 int set_stage_attributes(b200bssn_ctx* ctx) {
-  const int bytes = (int)StageCfg<ST, ADV>::kSmemBytes;
+  using Cfg = StageCfg<ST, ADV>;
   CK(ctx, cudaFuncSetAttribute(bssn_algebra_staged_kernel<ST, RK_NONE, ADV>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes(RK_NONE)));
   CK(ctx, cudaFuncSetAttribute(bssn_algebra_staged_kernel<ST, RK_FIRST, ADV>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes(RK_FIRST)));
   CK(ctx, cudaFuncSetAttribute(bssn_algebra_staged_kernel<ST, RK_MIDDLE, ADV>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes(RK_MIDDLE)));
   CK(ctx, cudaFuncSetAttribute(bssn_algebra_staged_kernel<ST, RK_LAST, ADV>,
-                               cudaFuncAttributeMaxDynamicSharedMemorySize, bytes));
+                               cudaFuncAttributeMaxDynamicSharedMemorySize, (int)Cfg::smem_bytes(RK_LAST)));
   return B200BSSN_OK;
 }
 
@@ -617,16 +617,16 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
     int alg_per_sm = 0;
     if (mx && !adv)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<float, RK_NONE, false>,
-                                                    StageCfg<float, false>::kThreads, StageCfg<float, false>::kSmemBytes);
+                                                    StageCfg<float, false>::kThreads, StageCfg<float, false>::smem_bytes(RK_NONE));
     else if (mx)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<float, RK_NONE, true>,
-                                                    StageCfg<float, true>::kThreads, StageCfg<float, true>::kSmemBytes);
+                                                    StageCfg<float, true>::kThreads, StageCfg<float, true>::smem_bytes(RK_NONE));
     else if (!adv)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<double, RK_NONE, false>,
-                                                    StageCfg<double, false>::kThreads, StageCfg<double, false>::kSmemBytes);
+                                                    StageCfg<double, false>::kThreads, StageCfg<double, false>::smem_bytes(RK_NONE));
     else
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<double, RK_NONE, true>,
-                                                    StageCfg<double, true>::kThreads, StageCfg<double, true>::kSmemBytes);
+                                                    StageCfg<double, true>::kThreads, StageCfg<double, true>::smem_bytes(RK_NONE));
     P->alg_grid = std::max(1, sms * std::max(1, alg_per_sm));
   }
 

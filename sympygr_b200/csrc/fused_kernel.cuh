@@ -167,6 +167,7 @@ __device__ __forceinline__ int fused_schedule(const FusedArgs& f, int& pending, 
 
 // Slots from this warp's shared-memory copy, KO sums straight from the ring in L2.
 struct FusedScratch {
+  static constexpr bool kHolds = false;
   const float* d;   // this lane's column: d[s * kStageW]
   const float* ko;  // this lane's KO sums in the ring: ko[v * 32]
   __device__ __forceinline__ float dv(int s) const { return d[s * kStageW]; }

@@ -127,6 +127,7 @@ const void* derivs_kernel(bool dd, bool closure) {
 
 template <typename ST>
 struct GlobalScratch {
+  static constexpr bool kHolds = false;
   const ST* d;       // slot 0 of the point
   __device__ __forceinline__ ST dv(int s) const { return __ldg(d + s * 32); }
   __device__ __forceinline__ double kov(int v) const { return (double)__ldg(d + (kKoSlot + v) * 32); }

@@ -28,6 +28,14 @@ namespace b200bssn {
 // derivatives: MIXED stages them too (2 warps per CTA, 3 CTAs per SM), FP64 reads them from
 // global memory like the second derivatives.
 constexpr int kStageW = 32;
+// RK4 stages that read the accumulator: their outputs are held back in shared memory until the
+// algebra is through, and the stage's update then follows for kUpdateBatch variables at a time.
+// Done output by output, each waited for its own load of the accumulator, which no compiler may
+// move ahead of the stores before it: an RK4 step on 64 blocks of 37^3 took 5.08 (MIXED) and 7.31
+// ms (FP64) instead of 4.46 and 6.63.  (The first stage, which writes the accumulator only,
+// gains nothing from it: 4.49 and 6.67 ms.)
+__host__ __device__ constexpr bool held_back(int mode) { return mode == RK_MIDDLE || mode == RK_LAST; }
+constexpr int kUpdateBatch = 8;
 template <typename ST, bool ADV = false>
 struct StageCfg {
   static constexpr int kSlots = num_slots(ADV);  // 234 / 162
@@ -39,8 +47,10 @@ struct StageCfg {
   static constexpr int kWarps = sizeof(ST) == 4 ? (ADV ? 2 : 4) : 1;
   static constexpr int kThreads = 32 * kWarps;
   static constexpr int kMinBlocks = sizeof(ST) == 4 ? (ADV ? 3 : 2) : 8;
-  static constexpr size_t kBytesPerWarp = (size_t)kStaged * kStageW * sizeof(ST);
-  static constexpr size_t kSmemBytes = kWarps * kBytesPerWarp;
+  // and the outputs that an RK4 stage holds back (held_back): in FP64 over the KO sums
+  static __host__ __device__ constexpr int slots(int mode) { return kStaged + (kAll && held_back(mode) ? kNumVars : 0); }
+  static __host__ __device__ constexpr size_t bytes_per_warp(int mode) { return (size_t)slots(mode) * kStageW * sizeof(ST); }
+  static __host__ __device__ constexpr size_t smem_bytes(int mode) { return kWarps * bytes_per_warp(mode); }
 };
 
 struct AlgebraArgs {
@@ -70,14 +80,28 @@ __device__ __forceinline__ double bc_asymptotic(int v) {
 // Derivative s of the algebra's numbering (72 first, 66 second, 72 advective); KO sums.
 __device__ __forceinline__ int deriv_slot(int s) { return s < kNumDerivs ? s : s + kNumVars; }
 
-template <typename ST, bool ALL>
+template <typename ST, bool ALL, int SLOTS>
 struct SharedScratch {
-  const ST* d;       // this lane's column: all slots, or the first 72 and the KO sums
+  static constexpr bool kHolds = true;
+  ST* d;             // this lane's column: all slots, or the first 72 and the KO sums
   const ST* g;       // this lane's slot 0 in the scratch
   __device__ __forceinline__ ST dv(int s) const {
     return ALL ? d[deriv_slot(s) * kStageW] : (s < 72 ? d[s * kStageW] : __ldg(g + deriv_slot(s) * kStageW));
   }
   __device__ __forceinline__ double kov(int v) const { return (double)d[((ALL ? kKoSlot : 72) + v) * kStageW]; }
+  // keeps output v of the algebra; the right-hand side that follows from it
+  __device__ __forceinline__ void hold(int v, ST val, double sigma) const {
+    if constexpr (ALL)
+      d[(SLOTS + v) * kStageW] = val;
+    else
+      d[(72 + v) * kStageW] = __dadd_rn(val, __dmul_rn(sigma, kov(v)));
+  }
+  __device__ __forceinline__ double held(int v, double sigma) const {
+    if constexpr (ALL)
+      return __dadd_rn((double)d[(SLOTS + v) * kStageW], __dmul_rn(sigma, kov(v)));
+    else
+      return d[(72 + v) * kStageW];
+  }
 };
 
 template <typename RT, class Src>
@@ -127,7 +151,10 @@ struct PointSink {
   template <typename RT>
   __device__ __forceinline__ void put(int v, RT val) {
     // rhs += sigma * (ko_x + ko_y + ko_z), rounded as rhs.cpp:332-369 rounds it
-    store_rhs<MODE>(*a, v, pp, __dadd_rn((double)val, __dmul_rn(a->ko_sigma, src.kov(v))), stage_in<MODE>(*a, v, pp));
+    if constexpr (held_back(MODE) && Src::kHolds)
+      src.hold(v, val, a->ko_sigma);
+    else
+      store_rhs<MODE>(*a, v, pp, __dadd_rn((double)val, __dmul_rn(a->ko_sigma, src.kov(v))), stage_in<MODE>(*a, v, pp));
   }
 };
 
@@ -277,7 +304,7 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
   constexpr int kPerPass = 32 / kPieces;                             // slots copied per instruction: 2 / 4
   extern __shared__ __align__(16) unsigned char s_stage[];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  ST* sd = reinterpret_cast<ST*>(s_stage + warp * Cfg::kBytesPerWarp);
+  ST* sd = reinterpret_cast<ST*>(s_stage + warp * Cfg::bytes_per_warp(MODE));
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(sd)) + 16u * (uint32_t)lane;
   const int nwarps = gridDim.x * Cfg::kWarps;
   // Neighbouring tasks share state and scratch lines and go to one CTA; fewer tasks than warps
@@ -330,9 +357,22 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
     cp_async_commit();
     cp_async_wait<0>();
     __syncwarp();  // the copies of every lane are visible to the whole warp
-    using Src = SharedScratch<ST, Cfg::kAll>;
+    using Src = SharedScratch<ST, Cfg::kAll, Cfg::kStaged>;
     const bool face = face_points<MODE>(a, B, p.i, p.j, p.k, p.valid, [sd, own](int l) { return Src{sd + l, own}; });
-    if (p.valid && !face) algebra_point_at<RT, MODE, Src, ADV>(a, B, p.i, p.j, p.k, Src{sd + lane, own});
+    if (p.valid && !face) {
+      const Src src{sd + lane, own};
+      algebra_point_at<RT, MODE, Src, ADV>(a, B, p.i, p.j, p.k, src);
+      if constexpr (held_back(MODE)) {
+#pragma unroll 1
+        for (int v0 = 0; v0 < kNumVars; v0 += kUpdateBatch) {
+          StageIn in[kUpdateBatch];
+#pragma unroll
+          for (int b = 0; b < kUpdateBatch; ++b) in[b] = stage_in<MODE>(a, v0 + b, pp);
+#pragma unroll
+          for (int b = 0; b < kUpdateBatch; ++b) store_rhs<MODE>(a, v0 + b, pp, src.held(v0 + b, a.ko_sigma), in[b]);
+        }
+      }
+    }
   }
 }
 
