@@ -772,17 +772,16 @@ def main():
                           peak32, tr.get("single_pass"), 1, peak_src)
             rl[mode] = {"single_pass": one, "evaluation": ev}
             continue
-        nchunks = max(1, plans[prec].launches // 3)  # 3 launches per chunk
         rl[mode] = {
             # derivative stage: reads the state over the padded blocks; its scratch is
             # not algorithmic (the reference's algorithm needs no scratch traffic)
-            "derivs": roofline(f"bssn_derivs_kind_kernel<{'float' if mode == 'mixed' else 'double'},*> (both kinds)",
+            "derivs": roofline(f"bssn_derivs_kind_kernel<{'float' if mode == 'mixed' else 'double'},*> (all launches)",
                                d_ms, npts, read_state, FLOPS_STENCIL, 0, hbm_peak, peak64, peak32,
-                               tr["derivs"], nchunks, peak_src),
+                               tr["derivs"], 1, peak_src),
             # algebra: the state at the point in, the 24 right-hand sides out
             "algebra": roofline(f"bssn_algebra_staged_kernel<{'float' if mode == 'mixed' else 'double'},0>",
                                 a_ms, npts, 2 * BYTES_VARS, f64_alg, f32_alg, hbm_peak, peak64, peak32,
-                                tr["algebra"], nchunks, peak_src),
+                                tr["algebra"], 1, peak_src),
             "evaluation": roofline(f"whole {mode} evaluation (all launches)",
                                    ms_mixed if mode == "mixed" else ms_fp64, npts,
                                    read_state + BYTES_VARS, FLOPS_STENCIL + f64_alg, f32_alg,

@@ -222,7 +222,7 @@ int b200bssn_check_finite(b200bssn_plan *plan, const double *const *arrays, uint
 /* Classic 4-stage Runge-Kutta over a plan's blocks (BSSN_RK4_STAGES = 4,
  * bssn/include/parameters.h:37; the reference repository itself has no
  * integrator).  The stage update runs in the epilogue of the algebra kernel, in
- * FP64 in both precisions, so a stage is the plan's two launches per chunk and the
+ * FP64 in both precisions, so a stage is the plan's launches and the
  * RHS never goes to memory.  The object owns three [24][span] FP64 buffers (the
  * accumulator and two stage states; span = the element range of the plan's
  * blocks).  Stage kernels write interior points only; ghost points of the stage

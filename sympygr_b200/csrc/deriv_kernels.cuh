@@ -235,7 +235,7 @@ struct RowsFor<float> { using type = SplitRows; };
 // the points 3, 4, 5 at a low face, 3..5 the points n-6, n-5, n-4 at a high one (closure_id).
 // A row reads the values m[k], k points from the face point inwards.  d1 and d2 sum five of
 // them in ascending index order, with the row's weights; ko sums from the far point inwards,
-// with weights by distance from the face.  Same operations and order as line_*: the weights
+// with weights by distance from the face.  Operations and order are the reference's: the weights
 // come from a table (in shared memory), so that lanes at different rows run one code.
 struct ClosureRow {
   double d1[5], d2[5];  // ascending index

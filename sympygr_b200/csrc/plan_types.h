@@ -13,7 +13,7 @@
 // rows of different tiles shared sectors, and the stores -- not the arithmetic, nor the
 // bytes -- set the derivative stage's time.  On 16 blocks of 69^3 (4.0 M points) the stage
 // took 1.43 ms (MIXED) and 2.00 ms (FP64), 0.67 and 0.72 ms with its stores switched off;
-// the same kernels storing whole sectors take 0.95 and 1.17 ms.
+// with whole sectors, and the rest of the rewrite, 0.83 and 1.14 ms.
 //
 // The algebra takes 32 points at a time along the block's rows (slab_point): two neighbouring
 // tiles' parts of a row, and, where a row has an odd number of tiles, its last part together
@@ -21,7 +21,8 @@
 // runs of up to 32 points, and no two warps share a sector of the scratch.  (Groups of four
 // points taken densely along the rows instead left fewer lanes idle, but on 135^3 blocks,
 // whose rows of 129 points then straddle the tiles or leave a group of one point, the algebra
-// took 1.64 instead of 1.23 ms, MIXED, and 2.69 instead of 2.16 ms, FP64, on 6.4 M points.)
+// took 1.64 instead of 1.38 ms, MIXED, and 2.69 instead of 2.38 ms, FP64, on 6.4 M points.
+// Two rows of one tile, whose 32 points are one block of the scratch: 1.52 and 2.46 ms.)
 #pragma once
 #include <stdint.h>
 

@@ -1,19 +1,15 @@
-// Finite-difference line operators of the reference's default build, evaluated on
-// values staged in shared memory.
+// Finite-difference operators of the reference's default build: the centred rows and the
+// scale factors of all rows (the closure rows are in deriv_kernels.cuh).
 //
-//   line_d1 : deriv64_{x,y,z}    bssn/src/derivs.cpp:2055-2434  6th-order centred first
-//                                                               derivative, 4th-order closures
-//   line_d2 : deriv64_{xx,yy,zz} bssn/src/derivs.cpp:2443-2833  6th-order centred second
-//                                                               derivative, 4th-order closures
-//   line_ko : ko_deriv42_{x,y,z} bssn/src/derivs.cpp:915-1319   Kreiss-Oliger operator
+//   d1 : deriv64_{x,y,z}    bssn/src/derivs.cpp:2055-2434  6th-order centred first derivative,
+//                                                          4th-order closures
+//   d2 : deriv64_{xx,yy,zz} bssn/src/derivs.cpp:2443-2833  6th-order centred second derivative,
+//                                                          4th-order closures
+//   ko : ko_deriv42_{x,y,z} bssn/src/derivs.cpp:915-1319   Kreiss-Oliger operator
 //
-// Each takes a pointer `p` to the value at the evaluation point, the element stride
-// `s` along the operator axis, the point's padded index `pos` on that axis, the
-// padded extent `n`, and whether the low/high face of that axis is a domain
-// boundary (bflag bits).  Closure rows replace the centred row within three points
-// of a flagged face; the high side wins where both apply, as the reference runs
-// its LEFT loop before its RIGHT loop.  Closure rows reach up to four points
-// inward; callers stage a 4-point halo.
+// Closure rows replace the centred row within three points of a flagged face (bflag bits);
+// the high side wins where both apply, as the reference runs its LEFT loop before its RIGHT
+// loop.
 //
 // Rounding: every product and sum is an explicitly rounded IEEE operation
 // (__dmul_rn/__dadd_rn, never contracted into an FMA) taken in the reference's
@@ -75,202 +71,9 @@ __device__ __forceinline__ double mad_rn(double acc, double c, double v) {
   return __dadd_rn(acc, __dmul_rn(c, v));
 }
 
-// Sum of coefficient[k] * value(offset[k]) in the given order (first term c0*v0).
-#define B2_T(c, k) __dmul_rn((c), p[(k) * s])
-#define B2_Q(c, k) __dmul_rn((c), q[(k) * s])
-
-__device__ __forceinline__ double line_d1(const double* p, int s, int pos, int n, bool lo,
-                                          bool hi, const LineScales& c) {
-  if (hi && pos >= n - 6) {
-    const int r = pos - (n - 6);
-    const double* q = p + (n - 4 - pos) * s;  // value at ie-1 = n-4; derivs.cpp:2132-2155
-    double a;
-    if (r == 0) {
-      a = B2_Q(1.0, -4);
-      a = __dadd_rn(a, B2_Q(-8.0, -3));
-      a = __dadd_rn(a, B2_Q(8.0, -1));
-      a = __dadd_rn(a, B2_Q(-1.0, 0));
-    } else if (r == 1) {
-      a = B2_Q(-1.0, -4);
-      a = __dadd_rn(a, B2_Q(6.0, -3));
-      a = __dadd_rn(a, B2_Q(-18.0, -2));
-      a = __dadd_rn(a, B2_Q(10.0, -1));
-      a = __dadd_rn(a, B2_Q(3.0, 0));
-    } else {
-      a = B2_Q(3.0, -4);
-      a = __dadd_rn(a, B2_Q(-16.0, -3));
-      a = __dadd_rn(a, B2_Q(36.0, -2));
-      a = __dadd_rn(a, B2_Q(-48.0, -1));
-      a = __dadd_rn(a, B2_Q(25.0, 0));
-    }
-    return __dmul_rn(a, c.d1_b);
-  }
-  if (lo && pos < 6) {
-    const int r = pos - 3;
-    const double* q = p - r * s;  // value at index 3; derivs.cpp:2094-2115
-    double a;
-    if (r == 0) {
-      a = B2_Q(-25.0, 0);
-      a = __dadd_rn(a, B2_Q(48.0, 1));
-      a = __dadd_rn(a, B2_Q(-36.0, 2));
-      a = __dadd_rn(a, B2_Q(16.0, 3));
-      a = __dadd_rn(a, B2_Q(-3.0, 4));
-    } else if (r == 1) {
-      a = B2_Q(-3.0, 0);
-      a = __dadd_rn(a, B2_Q(-10.0, 1));
-      a = __dadd_rn(a, B2_Q(18.0, 2));
-      a = __dadd_rn(a, B2_Q(-6.0, 3));
-      a = __dadd_rn(a, B2_Q(1.0, 4));
-    } else {
-      a = B2_Q(1.0, 0);
-      a = __dadd_rn(a, B2_Q(-8.0, 1));
-      a = __dadd_rn(a, B2_Q(8.0, 3));
-      a = __dadd_rn(a, B2_Q(-1.0, 4));
-    }
-    return __dmul_rn(a, c.d1_b);
-  }
-  double a = B2_T(-1.0, -3);
-  a = __dadd_rn(a, B2_T(9.0, -2));
-  a = __dadd_rn(a, B2_T(-45.0, -1));
-  a = __dadd_rn(a, B2_T(45.0, 1));
-  a = __dadd_rn(a, B2_T(-9.0, 2));
-  a = __dadd_rn(a, B2_T(1.0, 3));
-  return __dmul_rn(a, c.d1_c);
-}
-
-__device__ __forceinline__ double line_d2(const double* p, int s, int pos, int n, bool lo,
-                                          bool hi, const LineScales& c) {
-  if (hi && pos >= n - 6) {
-    const int r = pos - (n - 6);
-    const double* q = p + (n - 4 - pos) * s;  // derivs.cpp:2530-2551
-    double a;
-    if (r == 0) {
-      a = B2_Q(-1.0, -4);
-      a = __dadd_rn(a, B2_Q(16.0, -3));
-      a = __dadd_rn(a, B2_Q(-30.0, -2));
-      a = __dadd_rn(a, B2_Q(16.0, -1));
-      a = __dadd_rn(a, B2_Q(-1.0, 0));
-    } else if (r == 1) {
-      a = B2_Q(-1.0, -4);
-      a = __dadd_rn(a, B2_Q(4.0, -3));
-      a = __dadd_rn(a, B2_Q(6.0, -2));
-      a = __dadd_rn(a, B2_Q(-20.0, -1));
-      a = __dadd_rn(a, B2_Q(11.0, 0));
-    } else {
-      a = B2_Q(11.0, -4);
-      a = __dadd_rn(a, B2_Q(-56.0, -3));
-      a = __dadd_rn(a, B2_Q(114.0, -2));
-      a = __dadd_rn(a, B2_Q(-104.0, -1));
-      a = __dadd_rn(a, B2_Q(35.0, 0));
-    }
-    return __dmul_rn(a, c.d2_b);
-  }
-  if (lo && pos < 6) {
-    const int r = pos - 3;
-    const double* q = p - r * s;  // derivs.cpp:2490-2510
-    double a;
-    if (r == 0) {
-      a = B2_Q(35.0, 0);
-      a = __dadd_rn(a, B2_Q(-104.0, 1));
-      a = __dadd_rn(a, B2_Q(114.0, 2));
-      a = __dadd_rn(a, B2_Q(-56.0, 3));
-      a = __dadd_rn(a, B2_Q(11.0, 4));
-    } else if (r == 1) {
-      a = B2_Q(11.0, 0);
-      a = __dadd_rn(a, B2_Q(-20.0, 1));
-      a = __dadd_rn(a, B2_Q(6.0, 2));
-      a = __dadd_rn(a, B2_Q(4.0, 3));
-      a = __dadd_rn(a, B2_Q(-1.0, 4));
-    } else {
-      a = B2_Q(-1.0, 0);
-      a = __dadd_rn(a, B2_Q(16.0, 1));
-      a = __dadd_rn(a, B2_Q(-30.0, 2));
-      a = __dadd_rn(a, B2_Q(16.0, 3));
-      a = __dadd_rn(a, B2_Q(-1.0, 4));
-    }
-    return __dmul_rn(a, c.d2_b);
-  }
-  double a = B2_T(2.0, -3);
-  a = __dadd_rn(a, B2_T(-27.0, -2));
-  a = __dadd_rn(a, B2_T(270.0, -1));
-  a = __dadd_rn(a, B2_T(-490.0, 0));
-  a = __dadd_rn(a, B2_T(270.0, 1));
-  a = __dadd_rn(a, B2_T(-27.0, 2));
-  a = __dadd_rn(a, B2_T(2.0, 3));
-  return __dmul_rn(a, c.d2_c);
-}
-
-__device__ __forceinline__ double line_ko(const double* p, int s, int pos, int n, bool lo,
-                                          bool hi, const LineScales& c) {
-  if (hi && pos >= n - 6) {
-    const int r = pos - (n - 6);
-    const double* q = p + (n - 4 - pos) * s;  // derivs.cpp:1006-1028
-    double a;
-    if (r == 0) {
-      a = q[-5 * s];
-      a = __dadd_rn(a, B2_Q(-6.0, -4));
-      a = __dadd_rn(a, B2_Q(15.0, -3));
-      a = __dadd_rn(a, B2_Q(-19.0, -2));
-      a = __dadd_rn(a, B2_Q(12.0, -1));
-      a = __dadd_rn(a, B2_Q(-3.0, 0));
-      return __ddiv_rn(a, c.ko_s1);
-    } else if (r == 1) {
-      a = q[-4 * s];
-      a = __dadd_rn(a, B2_Q(-6.0, -3));
-      a = __dadd_rn(a, B2_Q(12.0, -2));
-      a = __dadd_rn(a, B2_Q(-10.0, -1));
-      a = __dadd_rn(a, B2_Q(3.0, 0));
-      return __ddiv_rn(a, c.ko_s2);
-    }
-    a = q[-3 * s];
-    a = __dadd_rn(a, B2_Q(-3.0, -2));
-    a = __dadd_rn(a, B2_Q(3.0, -1));
-    a = __dsub_rn(a, q[0]);
-    return __ddiv_rn(a, c.ko_s3);
-  }
-  if (lo && pos < 6) {
-    const int r = pos - 3;
-    const double* q = p - r * s;  // derivs.cpp:969-990 (summed from the far point inwards)
-    double a;
-    if (r == 0) {
-      a = q[3 * s];
-      a = __dadd_rn(a, B2_Q(-3.0, 2));
-      a = __dadd_rn(a, B2_Q(3.0, 1));
-      a = __dsub_rn(a, q[0]);
-      return __ddiv_rn(a, c.ko_s3);
-    } else if (r == 1) {
-      a = q[4 * s];
-      a = __dadd_rn(a, B2_Q(-6.0, 3));
-      a = __dadd_rn(a, B2_Q(12.0, 2));
-      a = __dadd_rn(a, B2_Q(-10.0, 1));
-      a = __dadd_rn(a, B2_Q(3.0, 0));
-      return __ddiv_rn(a, c.ko_s2);
-    }
-    a = q[5 * s];
-    a = __dadd_rn(a, B2_Q(-6.0, 4));
-    a = __dadd_rn(a, B2_Q(15.0, 3));
-    a = __dadd_rn(a, B2_Q(-19.0, 2));
-    a = __dadd_rn(a, B2_Q(12.0, 1));
-    a = __dadd_rn(a, B2_Q(-3.0, 0));
-    return __ddiv_rn(a, c.ko_s1);
-  }
-  double a = -p[-3 * s];
-  a = __dadd_rn(a, B2_T(6.0, -2));
-  a = __dadd_rn(a, B2_T(-15.0, -1));
-  a = __dadd_rn(a, B2_T(20.0, 0));
-  a = __dadd_rn(a, B2_T(-15.0, 1));
-  a = __dadd_rn(a, B2_T(6.0, 2));
-  a = __dsub_rn(a, p[3 * s]);
-  return __dmul_rn(c.ko_c, a);
-}
-
-#undef B2_T
-#undef B2_Q
-
 // Centred rows on a register window w[] (C = index of the evaluation point).
 // Callers invoke these inside fully unrolled loops, so every index folds to a
-// constant and the window stays in registers.  Same operations and order as the
-// centred branches above.
+// constant and the window stays in registers.
 template <int N>
 __device__ __forceinline__ double win_d1(const double (&w)[N], const int C,
                                          const LineScales& c) {
@@ -307,11 +110,6 @@ __device__ __forceinline__ double win_ko(const double (&w)[N], const int C,
   a = mad_rn(a, 6.0, w[C + 2]);
   a = __dsub_rn(a, w[C + 3]);
   return __dmul_rn(c.ko_c, a);
-}
-
-// True when the point at padded index `pos` takes a closure row.
-__device__ __forceinline__ bool closure_row(int pos, int n, bool lo, bool hi) {
-  return (lo && pos < 6) || (hi && pos >= n - 6);
 }
 
 }  // namespace b200bssn

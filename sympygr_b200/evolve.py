@@ -23,8 +23,8 @@ by ``--tiles``^3 blocks of padded size ``--tile-size`` around the same two punct
 the faces on the domain boundary carry the Sommerfeld values and one-sided closures
 (their bflag bits), the faces between blocks keep the frozen initial ghost data (the
 ghost exchange between blocks is outside this path).  dt = CFL * the smallest spacing.  The whole step loop runs as replays of a CUDA graph of
-``--graph-steps`` RK4 steps (each step: 4 stages x 3 launches per chunk, the stage
-update fused into the algebra kernel).  Every ``--check-every`` steps the driver
+``--graph-steps`` RK4 steps (each step: 4 stages of derivative and algebra launches per
+chunk, the stage update fused into the algebra kernel).  Every ``--check-every`` steps the driver
 evaluates the Hamiltonian and momentum constraints on the device (per-block sums of
 squares and maxima) and reads the lapse at the grid points nearest the two
 punctures.
