@@ -725,8 +725,9 @@ constexpr int kKindVars[2] = {13, 11};        // [DD]
 // first is launched as a programmatic dependent of the one before (launch_deriv), which lets
 // it start at once, so its CTAs fill the SMs as the ones before run out of items, and the
 // launches of a small plan run side by side.  A CTA ends only when the launch before has
-// ended, so that the last launch's end is the stage's.  (21^3 block, all faces flagged,
-// MIXED: 100 us in sequence, 149 us before the kernels and slabs changed.)
+// ended, so that the last launch's end is the stage's.  (A call on one 21^3 block with all
+// faces flagged, MIXED, whose launches last 20-30 us each, takes 80 us; 166 us before the
+// kernels, the slabs and this.)
 constexpr int kind_ctas_per_sm(bool dd, bool adv, int closure) {
   return dd ? (adv ? 4 : 6) : (closure == kClosureXY ? 6 : 8);
 }
