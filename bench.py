@@ -53,10 +53,10 @@ BYTES_VARS = 24 * 8
 # DRAM bytes per interior point of each kernel of an evaluation, from an ncu capture
 # (dram__bytes_read.sum + dram__bytes_write.sum) of a 3.15M-point case of the batch's
 # large blocks (four 69^3 and one 135^3, one flagged face): `python bench.py
-# --profile-case {mixed,fp64} [--single-pass]` (derivative stage: its two kernels summed;
+# --profile-case {mixed,fp64} [--single-pass]` (derivative stage: its kernels summed;
 # the one-pass kernel with its default 128-slot ring).
-NCU_TRAFFIC_PER_POINT = {"mixed": {"derivs": 375.0 + 646.0, "algebra": 1124.0, "single_pass": 836.0},
-                         "fp64": {"derivs": 580.0 + 1083.0, "algebra": 1897.0}}
+NCU_TRAFFIC_PER_POINT = {"mixed": {"derivs": 895.0, "algebra": 1409.0, "single_pass": 836.0},
+                         "fp64": {"derivs": 1573.0, "algebra": 1943.0}}
 REF_STEP_CAP, REF_WARMUP_CAP = 3, 1  # reference arm: ~32 s per full-batch step on 16 threads
 
 PG_TIMEOUT_S = 120  # process-group timeout under torchrun (N > 1)
