@@ -313,20 +313,39 @@ int64_t default_depth(const b200bssn_block* blocks, uint32_t nblocks, uint64_t c
 }
 
 // Orders each chunk's tiles by their closure rows (TileClosure), the longest first in each
-// list (cost ~ planes streamed).  The lists follow the blocks' face flags.
+// list (cost ~ planes streamed), and sizes the grids of the kernels that the lists call for.  The
+// lists follow the blocks' face flags.
 void order_tiles(b200bssn_plan* P) {
-  P->order.resize(P->tiles.size());
-  for (size_t k = 0; k < P->order.size(); ++k) P->order[k] = (int32_t)k;
-  for (ChunkRec& c : P->chunks) {
-    auto kind = [&](int32_t k) { return (int)tile_closure(P->blocks[P->tiles[k].block], P->tiles[k]); };
-    const auto lo = P->order.begin() + c.tile_begin, hi = lo + c.tile_count;
-    std::stable_sort(lo, hi, [&](int32_t x, int32_t y) {
-      const int kx = kind(x), ky = kind(y);
-      return kx != ky ? kx < ky : P->tiles[x].nz > P->tiles[y].nz;
-    });
-    for (int32_t& n : c.list) n = 0;
-    for (auto it = lo; it != hi; ++it) ++c.list[kind(*it)];
+  const size_t n = P->tiles.size();
+  std::vector<uint64_t> keys(n);  // list, planes descending, tile
+  for (size_t k = 0; k < n; ++k) {
+    const TileDev& t = P->tiles[k];
+    keys[k] = (uint64_t)tile_closure(P->blocks[t.block], t) << 56 | (uint64_t)(0xffffff - t.nz) << 32 | (uint64_t)k;
   }
+  P->order.resize(n);
+  bool any[3] = {};
+  for (ChunkRec& c : P->chunks) {
+    const auto lo = keys.begin() + c.tile_begin, hi = lo + c.tile_count;
+    std::sort(lo, hi);
+    for (int32_t& l : c.list) l = 0;
+    for (auto it = lo; it != hi; ++it) {
+      const int cl = (int)(*it >> 56);
+      ++c.list[cl];
+      any[cl] = true;
+      P->order[it - keys.begin()] = (int32_t)(*it & 0xffffffffu);
+    }
+  }
+  int sms = 0;
+  cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, P->ctx->device);
+  for (int k = 0; k < 2; ++k)
+    for (int cl = 0; cl < 3; ++cl) {
+      if (!any[cl] || P->deriv_grid[k][cl]) continue;
+      int per_sm = 0;
+      cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->kind_fn[k][cl], kItemThreads, 0);
+      // (the option counts CTAs of four warps)
+      if (P->deriv_ctas) per_sm = (int)std::min<int64_t>(per_sm, 2 * (int64_t)P->deriv_ctas);
+      P->deriv_grid[k][cl] = std::max(1, sms * std::max(1, per_sm));
+    }
 }
 
 int set_kernel_attributes(b200bssn_ctx* ctx) {
@@ -454,6 +473,7 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   P->ctx = ctx;
   P->precision = precision;
   P->advective = o.advective != 0;
+  P->deriv_ctas = o.deriv_ctas_per_sm;
   // The tuning knobs of earlier stencil kernels: the values they took are still accepted (the
   // kernels have one tile shape and register split now), the others still refused.
   {
@@ -606,14 +626,6 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   order_tiles(P);
   {
     const bool mx = precision == B200BSSN_MIXED, adv = P->advective;
-    for (int k = 0; k < 2; ++k)
-      for (int cl = 0; cl < 3; ++cl) {
-        int per_sm = 0;
-        cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, P->kind_fn[k][cl], kItemThreads, 0);
-        // (the option counts CTAs of four warps)
-        if (o.deriv_ctas_per_sm) per_sm = (int)std::min<int64_t>(per_sm, 2 * (int64_t)o.deriv_ctas_per_sm);
-        P->deriv_grid[k][cl] = std::max(1, sms * std::max(1, per_sm));
-      }
     int alg_per_sm = 0;
     if (mx && !adv)
       cudaOccupancyMaxActiveBlocksPerMultiprocessor(&alg_per_sm, bssn_algebra_staged_kernel<float, RK_NONE, false>,

@@ -86,7 +86,8 @@ struct b200bssn_plan {
   // the derivative kernels [kind: without / with second derivatives][TileClosure]
   // and their resident CTAs
   const void* kind_fn[2][3] = {};
-  int deriv_grid[2][3] = {};
+  int deriv_grid[2][3] = {};   // CTAs of each derivative kernel that a list calls for (0: none yet)
+  uint32_t deriv_ctas = 0;     // plan option deriv_ctas_per_sm
   int alg_grid = 0;           // resident CTAs of the persistent staged algebra kernel (MIXED)
   // one-pass path (MIXED, centred advection): tile-slabs in launch order, the
   // per-evaluation sync words and the scratch ring
