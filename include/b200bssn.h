@@ -119,8 +119,12 @@ int b200bssn_plan_destroy(b200bssn_plan *plan);
 /* Tuning knobs of a plan (0 in any field: the default). */
 typedef struct b200bssn_plan_options {
   uint64_t chunk_points;       /* interior points per kernel pair (scratch size) */
-  uint32_t slab_depth;         /* max interior z planes per work unit, but never fewer than 3
-                                * (default: by a cost model of the whole plan) */
+  uint32_t slab_depth;         /* max interior z planes per work unit, but never fewer than 3; fewer
+                                * where that many do not fit the largest scratch (default: by a cost
+                                * model of the whole plan).  A plan is refused with
+                                * B200BSSN_ERR_SIZE_LIMIT when a block's slab of this depth (48 by
+                                * default) holds 2^31 / 139 or more interior points (upwind mode:
+                                * 2^31 / 211). */
   uint32_t deriv_ctas_per_sm;  /* resident derivative warps per SM, in fours (default: as many as fit) */
   /* NULL, or one entry per block overriding slab_depth for that block (0: keep
    * slab_depth); lets a tuner pick the depth per block-size class. */

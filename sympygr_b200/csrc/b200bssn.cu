@@ -15,6 +15,7 @@
 #include "constraint_kernels.cuh"
 #include "fused_kernel.cuh"
 #include "plan_internal.h"
+#include "plan_layout.h"
 #include "rhs_kernels.cuh"
 
 using namespace b200bssn;
@@ -38,11 +39,6 @@ bool b200bssn::host::params_ok(const b200bssn_params* p) {
 
 namespace {
 
-constexpr int64_t kDefaultChunkPoints = int64_t(1) << 23;
-// scratch slots are addressed with 32-bit offsets: slots * scratch points < 2^31
-constexpr int64_t max_scratch_points(int slots) { return ((int64_t(1) << 31) / slots - 1) / kTilePlane * kTilePlane; }
-// the chunk sizes accepted (interior points; the limit of a scratch without padding)
-constexpr int64_t max_chunk_points(bool adv) { return (int64_t(1) << 31) / (kNumDerivs + (adv ? 3 * kNumVars : 0) + 1) - 1; }
 // work counters of an evaluation, zeroed at its start: one per derivative launch of a chunk
 constexpr size_t kDerivCounters = 6;
 constexpr size_t counter_words(size_t chunks) { return kDerivCounters * chunks; }
@@ -279,39 +275,6 @@ int b200bssn::host::launch_plan(b200bssn_plan* P, double* const* rhs, const doub
 
 namespace {
 
-// Default z-slab depth of a plan, from a model of the derivative stage: a tile costs its
-// planes, the 6 halo planes and about 4 planes' worth of start-up; the 11 variables with second
-// derivatives (the longer kernel) share out 6 CTAs per SM, and each launch ends with one
-// tile's time.  Deep slabs pay the halo less often, shallow ones give small plans enough
-// items and every launch a shorter tail.  (16 blocks of 69^3 as one slab each, or in slabs of
-// 48, 24, 12, 6, 3 planes, MIXED: 0.86, 0.91, 0.93, 1.07, 1.32, 1.76 ms.)
-int64_t default_depth(const b200bssn_block* blocks, uint32_t nblocks, uint64_t chunk_points, int sms) {
-  const double resident = 6.0 * std::max(1, sms);
-  const int64_t capacity = chunk_points ? (int64_t)chunk_points : kDefaultChunkPoints;
-  int64_t best = 3;
-  double best_cost = 0.0;
-  for (const int64_t depth : {3, 4, 5, 6, 8, 11, 16, 22, 33, 44, 66, 99, 132}) {
-    double work = 0.0, points = 0.0;
-    int64_t longest = 0;
-    for (uint32_t b = 0; b < nblocks; ++b) {
-      const int64_t I0 = (int64_t)blocks[b].sz[0] - 6, I1 = (int64_t)blocks[b].sz[1] - 6, I2 = (int64_t)blocks[b].sz[2] - 6;
-      if (I0 < 7 || I1 < 7 || I2 < 7) continue;  // refused later
-      const int64_t n = std::min((I2 + depth - 1) / depth, I2 / 3);
-      const int64_t tiles = ((I0 + kTileX - 1) / kTileX) * ((I1 + kTileY - 1) / kTileY);
-      work += (double)tiles * (double)(I2 + 10 * n);
-      points += (double)I0 * I1 * I2;
-      longest = std::max(longest, (I2 + n - 1) / n + 10);
-    }
-    const double launches = std::max(1.0, points / (double)capacity);
-    const double cost = work * kKindVars[1] / resident + launches * (double)longest;
-    if (best_cost == 0.0 || cost < best_cost) {
-      best_cost = cost;
-      best = depth;
-    }
-  }
-  return best;
-}
-
 // Orders each chunk's tiles by their closure rows (TileClosure), the longest first in each
 // list (cost ~ planes streamed), and sizes the grids of the kernels that the lists call for.  The
 // lists follow the blocks' face flags.
@@ -464,7 +427,6 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   b200bssn_plan_options o;
   std::memset(&o, 0, sizeof(o));
   if (opts) o = *opts;
-  const uint64_t chunk_points = o.chunk_points;
   if (!ctx || !blocks || !out || nblocks == 0) return B200BSSN_ERR_INVALID_ARGUMENT;
   if (precision != B200BSSN_FP64 && precision != B200BSSN_MIXED) return B200BSSN_ERR_INVALID_ARGUMENT;
   *out = nullptr;
@@ -491,12 +453,9 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
   else
     P->advective ? kind_kernels<double, true>(P->kind_fn) : kind_kernels<double, false>(P->kind_fn);
   const int nslots = num_slots(P->advective);
-  const int64_t kMaxChunkPoints = max_chunk_points(P->advective), kMaxScratch = max_scratch_points(nslots);
   int sms = 0;
   cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, ctx->device);
-  const int64_t slab_depth = o.slab_depth ? (int64_t)o.slab_depth : default_depth(blocks, nblocks, chunk_points, sms);
   P->span_lo = UINT64_MAX;
-  int64_t max_slab = 0;  // interior points
   for (uint32_t b = 0; b < nblocks; ++b) {
     const b200bssn_block& in = blocks[b];
     for (int a = 0; a < 3; ++a) {
@@ -526,77 +485,15 @@ int b200bssn_plan_create_ex(b200bssn_ctx* ctx, const b200bssn_block* blocks, uin
     P->span_lo = std::min<uint64_t>(P->span_lo, in.offset);
     P->span_hi = std::max<uint64_t>(P->span_hi, in.offset + npad);
     const int64_t I0 = in.sz[0] - 6, I1 = in.sz[1] - 6, I2 = in.sz[2] - 6;
-    // z-slabs of nearly equal depth (<= depth planes, and never below three, see cut_start):
-    // the derivative kernels stream each slab plus 3 halo planes on each side
-    const int64_t depth = (o.block_slab_depth && o.block_slab_depth[b])
-                              ? (int64_t)o.block_slab_depth[b] : slab_depth;
-    const int64_t nslab = std::min((I2 + depth - 1) / depth, I2 / 3);
-    if ((uint64_t)I0 * I1 * ((I2 + nslab - 1) / nslab) > (uint64_t)INT32_MAX) {
-      delete P;
-      return B200BSSN_ERR_INVALID_ARGUMENT;
-    }
-    for (int64_t sl = 0; sl < nslab; ++sl) {
-      const int64_t k0 = sl * I2 / nslab, k1 = (sl + 1) * I2 / nslab;
-      P->slabs.push_back({(int32_t)b, (int32_t)k0, (int32_t)(k1 - k0), 0});
-      max_slab = std::max<int64_t>(max_slab, I0 * I1 * (k1 - k0));
-    }
     P->points += (uint64_t)(I0 * I1 * I2);
   }
-  int64_t capacity = chunk_points ? (int64_t)chunk_points : kDefaultChunkPoints;
-  capacity = std::min(std::max(capacity, max_slab), kMaxChunkPoints);
-  if (max_slab > kMaxChunkPoints) {
-    delete P;
-    return B200BSSN_ERR_SIZE_LIMIT;
-  }
-  // pack slabs into chunks
-  ChunkRec cur{0, 0, {0, 0, 0}, 0, 0, 0};
-  int64_t used = 0;  // scratch points of the current chunk
-  auto flush = [&]() {
-    if (cur.points > 0) {
-      cur.tile_count = (int32_t)P->tiles.size() - cur.tile_begin;
-      cur.range_count = (int32_t)P->ranges.size() - cur.range_begin;
-      P->chunks.push_back(cur);
-      P->cap = std::max<int64_t>(P->cap, used);
-    }
-    cur = ChunkRec{(int32_t)P->tiles.size(), 0, {0, 0, 0}, (int32_t)P->ranges.size(), 0, 0};
-    used = 0;
-  };
-  for (size_t si = 0; si < P->slabs.size(); ++si) {
-    SlabDev& u = P->slabs[si];
-    const BlockDev& B = P->blocks[u.block];
-    const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6;
-    const int cutx = num_cuts(I0, kTileX), cuty = num_cuts(I1, kTileY);
-    const int64_t points = (int64_t)I0 * I1 * u.nz, need = (int64_t)cutx * cuty * u.nz * kTilePlane;
-    if (need > kMaxScratch) {
+  {
+    const int rc = lay_out(*P, blocks, P->blocks, o, max_scratch_points(nslots), sms);
+    if (rc != B200BSSN_OK) {
       delete P;
-      return B200BSSN_ERR_SIZE_LIMIT;
+      return rc;
     }
-    // a block's slabs stay in one chunk when the whole block fits in one
-    const int64_t block_pts = (int64_t)I0 * I1 * (B.sz[2] - 6);
-    const bool first = si == 0 || P->slabs[si - 1].block != u.block;
-    if (first && block_pts <= capacity && cur.points + block_pts > capacity) flush();
-    if (cur.points + points > capacity || used + need > kMaxScratch) flush();
-    cur.points += points;
-    u.sbase = (int32_t)used;
-    for (int ty = 0; ty < cuty; ++ty)
-      for (int tx = 0; tx < cutx; ++tx) {
-        TileDev t;
-        t.block = u.block;
-        t.sbase = u.sbase + (ty * cutx + tx) * u.nz * kTilePlane;
-        t.k0 = u.k0;
-        t.nz = u.nz;
-        t.i0 = (int16_t)cut_start(I0, kTileX, tx);
-        t.j0 = (int16_t)cut_start(I1, kTileY, ty);
-        t.ex = (int16_t)(cut_start(I0, kTileX, tx + 1) - t.i0);
-        t.ey = (int16_t)(cut_start(I1, kTileY, ty + 1) - t.j0);
-        P->tiles.push_back(t);
-      }
-    used += need;
-    const int tasks = (int)slab_tasks(B, u.nz);
-    for (int s = 0; s < tasks; s += kRangeTasks)
-      P->ranges.push_back({(int32_t)si, s, std::min(kRangeTasks, tasks - s)});
   }
-  flush();
   // Host pipeline partition: chunk c owns elements [part[c], part[c+1]) when the
   // chunks' blocks are disjoint and in increasing offset order.
   {

@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "b200bssn.h"
+#include "plan_layout.h"
 #include "plan_types.h"
 
 namespace b200bssn {
@@ -16,6 +17,7 @@ struct ConstraintArgs;
 }  // namespace b200bssn
 
 using b200bssn::BlockDev;
+using b200bssn::ChunkRec;
 using b200bssn::RangeDev;
 using b200bssn::SlabDev;
 using b200bssn::TileDev;
@@ -41,25 +43,13 @@ struct b200bssn_ctx {
   cudaEvent_t blk_ev[b200bssn::kNumVars] = {};
 };
 
-struct ChunkRec {
-  int32_t tile_begin, tile_count;
-  int32_t list[3];  // how many of them take which closure rows (TileClosure): `order` holds them so
-  int32_t range_begin, range_count;
-  int64_t points;
-};
-
-struct b200bssn_plan {
+struct b200bssn_plan : b200bssn::PlanLayout {
   b200bssn_ctx* ctx = nullptr;
   uint32_t precision = 0;
   bool advective = false;  // upwind mode: 72 more scratch slots (advective derivatives)
   std::vector<BlockDev> blocks;
-  std::vector<SlabDev> slabs;
-  std::vector<TileDev> tiles;
   std::vector<int32_t> order;  // per chunk its tiles in the order the derivative kernels take them
-  std::vector<RangeDev> ranges;
-  std::vector<ChunkRec> chunks;
   uint64_t points = 0;
-  int64_t cap = 0;  // scratch points of a buffer
   uint64_t span_lo = 0, span_hi = 0;  // element range touched in the variable arrays
   // device
   void* desc = nullptr;  // blocks | slabs | tiles | order | ranges

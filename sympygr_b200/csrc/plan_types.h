@@ -69,7 +69,15 @@ struct SlabDev {
   int32_t block;
   int32_t k0, nz;     // first interior plane (0-based interior index), planes
   int32_t sbase;      // first scratch point of the slab within its chunk (a multiple of 128)
+  // a strip of the planes' rows (whole tiles) where the planes are too large for the scratch:
+  // first row, and how many of the block's rows it leaves out
+  int32_t j0 = 0, jcut = 0;
 };
+// tile rows of a slab: the first one's number in the block, and how many
+__host__ __device__ inline int first_cut(const SlabDev& s) { return (s.j0 + kTileY / 2) / kTileY; }
+__host__ __device__ inline int cut_rows(int n, const SlabDev& s) {
+  return cut_of(n, kTileY, s.j0 + n - s.jcut - 1) - first_cut(s) + 1;
+}
 
 // A column tile of a slab.
 struct TileDev {
@@ -99,14 +107,14 @@ __host__ __device__ inline RowTasks row_tasks(int I0) {
   const int lanes = (I0 - cut_start(I0, kTileX, tiles - 1) + kGroup - 1) / kGroup * kGroup, rows = 32 / lanes;
   return {tiles, pairs, lanes, rows, rows * pairs + 1};
 }
-// Tasks of a slab of nz planes of block B.
-__host__ __device__ inline int64_t slab_tasks(const BlockDev& B, int nz) {
+// Tasks of a slab of nz planes of block B that leaves out jcut of its rows.
+__host__ __device__ inline int64_t slab_tasks(const BlockDev& B, int nz, int jcut = 0) {
   const RowTasks t = row_tasks(B.sz[0] - 6);
-  return ((int64_t)(B.sz[1] - 6) * nz + t.rows - 1) / t.rows * t.tasks;
+  return ((int64_t)(B.sz[1] - 6 - jcut) * nz + t.rows - 1) / t.rows * t.tasks;
 }
 // The point of lane `lane` of a task of slab s.
 __host__ __device__ inline SlabPoint slab_point(const BlockDev& B, const SlabDev& s, int task, int lane) {
-  const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6, rows = I1 * s.nz;
+  const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6, J = I1 - s.jcut, rows = J * s.nz;
   const RowTasks t = row_tasks(I0);
   const int set = task / t.tasks, k = task - set * t.tasks;
   int r = set * t.rows, cx, x;  // row, its tile, point in the tile
@@ -124,9 +132,9 @@ __host__ __device__ inline SlabPoint slab_point(const BlockDev& B, const SlabDev
   const int x0 = cut_start(I0, kTileX, cx);
   const bool valid = r < rows && x0 + x < cut_start(I0, kTileX, cx + 1);
   r = r < rows ? r : rows - 1;
-  const int z = r / I1, y = r - z * I1, cy = cut_of(I1, kTileY, y);
+  const int z = r / J, y = s.j0 + r - z * J, cy = cut_of(I1, kTileY, y);
   return {3 + x0 + x, 3 + y, 3 + s.k0 + z,
-          s.sbase + ((cy * t.tiles + cx) * s.nz + z) * kTilePlane + row_off(y - cut_start(I1, kTileY, cy)) + x, valid};
+          s.sbase + (((cy - first_cut(s)) * t.tiles + cx) * s.nz + z) * kTilePlane + row_off(y - cut_start(I1, kTileY, cy)) + x, valid};
 }
 
 // Which closure rows a tile's output points take: those within three points of a flagged face.
