@@ -261,7 +261,7 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
         // the run's slots are in shared memory: drop their lines from L2 unwritten
         for (int q = lane; q < (int)(kFusedStageBytes / 128); q += 32)
           discard_l2_line(reinterpret_cast<const char*>(gd) + 128 * q);
-        const bool face = face_points<MODE>(f.a, B, i, j, k, valid, [&](int l) { return FusedScratch{sd + l, gk + l}; });
+        const bool face = face_points<MODE, kFaceBatch<float, MODE>>(f.a, B, i, j, k, valid, [&](int l) { return FusedScratch{sd + l, gk + l}; });
         if (valid && !face) algebra_point_at<float, MODE, FusedScratch, false>(f.a, B, i, j, k, FusedScratch{sd + lane, gk + lane});
         __syncwarp();  // every lane has read its KO sums
         if (lane < kNumVars) discard_l2_line(gk + lane * 32);

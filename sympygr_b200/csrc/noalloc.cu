@@ -156,7 +156,7 @@ noalloc_algebra(const __grid_constant__ AlgebraArgs a, const __grid_constant__ N
   const int lp = start + (valid ? threadIdx.x : 0), r = lp / t.ex, z = r / t.ey;
   const int i = 3 + t.i0 + (lp - r * t.ex), j = 3 + t.j0 + (r - z * t.ey), k = 3 + t.k0 + z;
   const ST* const scr = static_cast<const ST*>(a.scr);
-  const bool face = face_points<RK_NONE>(a, g.block, i, j, k, valid, [&](int l) {
+  const bool face = face_points<RK_NONE, kFaceBatch<ST, RK_NONE>>(a, g.block, i, j, k, valid, [&](int l) {
     return GlobalScratch<ST>{scr + scr_index<NS>(0, __shfl_sync(0xffffffffu, t.sbase + lp, l))};
   });
   if (valid && !face)

@@ -186,12 +186,18 @@ __device__ __forceinline__ PointPos point_pos(const BlockDev& B, int i, int j, i
 // A row meets the two x faces with one point each, so nearly every warp of a flagged block has
 // one such lane, and its 24 variables one after another -- a load from L2 and a chain of
 // FP64 operations each -- took as long as the algebra of all the others.  The (face point,
-// variable) pairs are therefore shared out over the lanes, kFaceBatch loads in flight per lane.
+// variable) pairs are therefore shared out over the lanes, BATCH of them in flight per lane.
 // Per evaluation of 64 blocks of 37^3 with all faces flagged (1.9 M points) the algebra took
 // 0.91 ms (MIXED) and 1.19 ms (FP64) with each lane looping over its own variables, 0.43 and
 // 0.69 ms without faces; so shared out 0.49 and 0.76 ms.
-constexpr int kFaceBatch = 4;
-template <int MODE, class At>
+// In FP64, at 255 registers, what a batch holds is paid for in spills of the whole kernel: with
+// batches of four the RK4 stages spilled 144-268 bytes per thread, with one 24-48; the plain
+// right-hand side 72, with two 40; the upwind mode 376, with two 312.  An RK4 step on 50 blocks
+// of 37^3 takes 7 % less with batches of one than of four (6 % with all faces flagged), a
+// right-hand side 4 % less with batches of two.
+template <typename ST, int MODE>
+constexpr int kFaceBatch = sizeof(ST) == 4 ? 4 : (MODE == RK_NONE ? 2 : 1);
+template <int MODE, int BATCH, class At>
 __device__ __forceinline__ bool face_points(const AlgebraArgs& a, const BlockDev& B, int i, int j, int k, bool valid,
                                             const At& at) {
   if (B.bflag == 0) return false;
@@ -209,13 +215,13 @@ __device__ __forceinline__ bool face_points(const AlgebraArgs& a, const BlockDev
   const int64_t pp = B.offset + i + (int64_t)B.sz[0] * (j + (int64_t)B.sz[1] * k);
   const int dv = 32 / n, dq = 32 - dv * n;
   int v = lane / n, q = lane - v * n;  // this lane's variable and face point
-  for (int pass = 0; pass < (kNumVars * n + 31) / 32; pass += kFaceBatch) {
-    int va[kFaceBatch], from[kFaceBatch];
-    int64_t pa[kFaceBatch];
-    double f[kFaceBatch], d[kFaceBatch][3], ko[kFaceBatch];
-    StageIn in[kFaceBatch];
+  for (int pass = 0; pass < (kNumVars * n + 31) / 32; pass += BATCH) {
+    int va[BATCH], from[BATCH];
+    int64_t pa[BATCH];
+    double f[BATCH], d[BATCH][3], ko[BATCH];
+    StageIn in[BATCH];
 #pragma unroll
-    for (int b = 0; b < kFaceBatch; ++b) {
+    for (int b = 0; b < BATCH; ++b) {
       from[b] = __shfl_sync(0xffffffffu, owner, q);
       pa[b] = __shfl_sync(0xffffffffu, pp, from[b]);
       const auto src = at(from[b]);
@@ -232,7 +238,7 @@ __device__ __forceinline__ bool face_points(const AlgebraArgs& a, const BlockDev
       if (q >= n) q -= n, ++v;
     }
 #pragma unroll
-    for (int b = 0; b < kFaceBatch; ++b) {
+    for (int b = 0; b < BATCH; ++b) {
       const double x = __shfl_sync(0xffffffffu, P.x, from[b]), y = __shfl_sync(0xffffffffu, P.y, from[b]);
       const double z = __shfl_sync(0xffffffffu, P.z, from[b]), ir = __shfl_sync(0xffffffffu, inv_r, from[b]);
       if (va[b] < kNumVars) {
@@ -358,7 +364,7 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
     cp_async_wait<0>();
     __syncwarp();  // the copies of every lane are visible to the whole warp
     using Src = SharedScratch<ST, Cfg::kAll, Cfg::kStaged>;
-    const bool face = face_points<MODE>(a, B, p.i, p.j, p.k, p.valid, [sd, own](int l) { return Src{sd + l, own}; });
+    const bool face = face_points<MODE, kFaceBatch<ST, MODE>>(a, B, p.i, p.j, p.k, p.valid, [sd, own](int l) { return Src{sd + l, own}; });
     if (p.valid && !face) {
       const Src src{sd + lane, own};
       algebra_point_at<RT, MODE, Src, ADV>(a, B, p.i, p.j, p.k, src);
