@@ -288,12 +288,14 @@ __device__ __forceinline__ double closure_ko(const double (&m)[6], int id, const
   return __ddiv_rn(a, dist == 0 ? sc.ko_s3 : (dist == 1 ? sc.ko_s2 : sc.ko_s1));
 }
 
-// Where an item's outputs go.  FULL: a tile of the plan's scratch (128 scratch points per
-// plane, whole sectors stored: the lanes that pad a row write values nobody reads).  Else
-// points numbered densely (the allocation-free entry point, whose fixed array has no room
-// for the padding): lp = base + tx + row_stride * ty + plane_pts * plane.
+// Where an item's outputs go.  FULL: a tile of the plan's scratch (planes 128 scratch points
+// apart, rows by point_off; whole sectors stored: the lanes that pad a row write values
+// nobody reads).  Else points numbered densely (the allocation-free entry point, whose fixed
+// array has no room for the padding): lp = base + tx + row_stride * ty + plane_pts * plane.
 struct ScratchMap {
-  int32_t base, row_stride, plane_pts;
+  int32_t base;
+  bool narrow;
+  int32_t row_stride, plane_pts;
 };
 
 // Planes per loop pass (measured on 16 blocks of 69^3, MIXED / FP64 ms: without second
@@ -407,8 +409,8 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
   ST* const sd_ko = static_cast<ST*>(a.scr) + (kKoSlot + v) * 32;                // KO sum
   ST* const sd_adv = static_cast<ST*>(a.scr) + (kAdvSlot + 3 * v) * 32;          // upwind mode
   auto col = [](int lp) { return (lp >> 5) * (NS * 32) + (lp & 31); };
-  const int full0 = col(sm.base + row_off(ty0) + tx);
-  static_assert(kRows == 2, "row_off puts a thread's second row 32 scratch points after its first");
+  const int full0 = col(sm.base + point_off(sm.narrow, tx, ty0));
+  static_assert(kRows == 2, "point_off puts a thread's second row 32 scratch points after its first");
   const int lp0 = sm.base + tx + sm.row_stride * ty0;
   auto at = [&](int r, int o) {
     if constexpr (FULL) return full0 + o * (kTilePlane / 32 * NS * 32) + r * (NS * 32);
@@ -444,7 +446,7 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
 
   // upwind mode: the sign bits of the thread's points, read one plane ahead (up_next); the
   // last four planes' in up_bits, the newest lowest
-  const uint8_t* const up0 = ADV ? a.up + sm.base + row_off(ty0) + tx : nullptr;
+  const uint8_t* const up0 = ADV ? a.up + sm.base + point_off(sm.narrow, tx, ty0) : nullptr;
   uint32_t up_bits[R] = {}, up_next[R] = {};
   auto load_up = [&](int o) {
 #pragma unroll
@@ -697,10 +699,11 @@ bssn_shift_signs_kernel(const double* b0, const double* b1, const double* b2, co
   const TileDev t = tiles[blockIdx.x];
   const BlockDev& B = blocks[t.block];
   const int x = threadIdx.x % kTileX, y = threadIdx.x / kTileX;
-  if (y >= t.ey) return;
+  const bool narrow = t.ex <= kNarrow;
+  if (y >= t.ey || (narrow && x >= kNarrow)) return;
   const int64_t plane = (int64_t)B.sz[0] * B.sz[1];
   int64_t p = B.offset + (3 + t.i0 + min(x, t.ex - 1)) + (int64_t)B.sz[0] * (3 + t.j0 + y) + plane * (3 + t.k0);
-  uint8_t* const out = up + t.sbase + row_off(y) + x;
+  uint8_t* const out = up + t.sbase + point_off(narrow, x, y);
 #pragma unroll 4
   for (int z = 0; z < t.nz; ++z, p += plane)
     out[z * kTilePlane] = (uint8_t)((__ldg(b0 + p) > 0.0) | (__ldg(b1 + p) > 0.0) << 1 | (__ldg(b2 + p) > 0.0) << 2);
@@ -750,7 +753,7 @@ bssn_derivs_kind_kernel(const __grid_constant__ DerivArgs a) {
     const int item = s_item;
     if (item >= a.tile_count * NV) break;
     const TileDev t = a.tiles[a.order[item / NV]];
-    const ScratchMap sm{t.sbase, 0, 0};
+    const ScratchMap sm{t.sbase, t.ex <= kNarrow, 0, 0};
     derive_item<ST, DD, ADV, CLOSURE, true>(a, a.blocks[t.block], t, sm, kind_var(DD, item % NV), S, s_closure,
                                         reinterpret_cast<ClosureValues*>(s_fix), 1);
   }

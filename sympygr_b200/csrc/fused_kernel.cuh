@@ -208,7 +208,7 @@ bssn_fused_kernel(const __grid_constant__ FusedArgs f) {
       const int T = idx / kFusedItems, v = kFusedItemVars * (idx % kFusedItems) + half;
       const FusedTileDev ft = f.tiles[T];
       const TileDev t{ft.block, 0, ft.k0, ft.nz, ft.i0, ft.j0, ft.ex, ft.ey};
-      const ScratchMap sm{(T % f.nring) * kFusedSlotPts, 0, 0};
+      const ScratchMap sm{(T % f.nring) * kFusedSlotPts, false, 0, 0};
       const bool cl = tile_closure(f.d.blocks[ft.block], t) != kClosureNone;
       if (dd_index(v) >= 0) {
         if (cl)

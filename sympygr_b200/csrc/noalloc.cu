@@ -112,7 +112,7 @@ noalloc_derivs(const __grid_constant__ DerivArgs a, const __grid_constant__ Noal
     __syncthreads();
   }
   const TileDev t = noalloc_tile(g, blockIdx.x / NV);
-  const ScratchMap sm{t.sbase, t.ex, t.ex * t.ey};
+  const ScratchMap sm{t.sbase, false, t.ex, t.ex * t.ey};
   derive_item<ST, DD, false, CLOSURE, false>(a, g.block, t, sm, kind_var(DD, blockIdx.x % NV), S, s_closure,
                                              reinterpret_cast<ClosureValues*>(s_fix), 1);
   asm volatile("griddepcontrol.wait;" ::: "memory");

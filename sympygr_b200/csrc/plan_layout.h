@@ -34,12 +34,17 @@ struct PlanLayout {
   int64_t cap = 0;  // scratch points of a buffer
 };
 
-// Interior extents of a block and the scratch points of one of its planes.
+// Interior extents of a block, its rows and columns of tiles, and the scratch points of a plane.
 struct Interior {
-  int64_t n[3], plane;
+  int64_t n[3];
+  int cutx, cuty;
+  int64_t plane;
   explicit Interior(const b200bssn_block& b) : n{(int64_t)b.sz[0] - 6, (int64_t)b.sz[1] - 6, (int64_t)b.sz[2] - 6} {
-    plane = ((n[0] + kTileX - 1) / kTileX) * ((n[1] + kTileY - 1) / kTileY) * kTilePlane;
+    cutx = num_cuts((int)n[0], kTileX);
+    cuty = num_cuts((int)n[1], kTileY);
+    plane = (int64_t)cutx * cuty * kTilePlane;
   }
+  bool narrow() const { return n[0] - cut_start((int)n[0], kTileX, cutx - 1) <= kNarrow; }  // the last column of tiles
   int64_t points(int64_t planes) const { return n[0] * n[1] * planes; }
   // Slabs of nearly equal depth, of at most `depth` planes and `limit` scratch points each but
   // never fewer than three planes (see cut_start).
@@ -66,7 +71,7 @@ inline int64_t default_depth(const b200bssn_block* blocks, size_t nblocks, int64
     for (size_t b = 0; b < nblocks; ++b) {
       const Interior in(blocks[b]);
       const int64_t n = in.slabs(depth, limit);
-      work += (double)(in.plane / kTilePlane) * (double)(in.n[2] + 10 * n);
+      work += (double)(in.cutx * in.cuty) * (double)(in.n[2] + 10 * n);
       points += (double)in.points(in.n[2]);
       longest = std::max(longest, (in.n[2] + n - 1) / n + 10);
     }
@@ -108,12 +113,12 @@ inline int lay_out(PlanLayout& L, const b200bssn_block* blocks, const std::vecto
     const int64_t n = in.slabs(depth_asked(b) ? depth_asked(b) : model_depth, max_scratch);
     for (int64_t sl = 0; sl < n; ++sl) {
       const int64_t k0 = sl * in.n[2] / n, nz = (sl + 1) * in.n[2] / n - k0;
-      const int I1 = (int)in.n[1], cuts = num_cuts(I1, kTileY);
-      const int64_t row = in.plane / cuts * nz;  // scratch points of a row of tiles
-      const int per = row * cuts <= max_scratch ? cuts : (int)(max_scratch / row);
-      for (int c = 0; c < cuts; c += per) {
-        const int j0 = cut_start(I1, kTileY, c), j1 = cut_start(I1, kTileY, std::min(c + per, cuts));
-        L.slabs.push_back({(int32_t)b, (int32_t)k0, (int32_t)nz, 0, j0, I1 - (j1 - j0)});
+      int per = in.cuty;  // rows of tiles per strip
+      if (in.plane * nz > max_scratch) per = (int)std::max<int64_t>(1, max_scratch / (in.cutx * kTilePlane * nz));
+      const int I1 = (int)in.n[1];
+      for (int c = 0; c < in.cuty; c += per) {
+        const int j0 = cut_start(I1, kTileY, c), j1 = cut_start(I1, kTileY, std::min(c + per, in.cuty));
+        L.slabs.push_back({(int32_t)b, (int32_t)k0, (int32_t)nz, 0, j0, I1 - (j1 - j0), in.narrow()});
       }
     }
   }

@@ -7,8 +7,9 @@
 // algebra launch (runs of points along the block's rows).
 //
 // Scratch points.  Every tile owns 128 scratch points per plane, planes one after another;
-// row y of the tile sits at row_off(y), 16 points.  So a store of the derivative stage fills
-// whole 32-byte sectors, and a 32-point block of the scratch (scr_index) belongs to one tile.
+// row y of the tile sits at row_off(y), 16 points (narrow tiles: see kNarrow).  So a store of
+// the derivative stage fills whole 32-byte sectors, and a 32-point block of the scratch
+// (scr_index) belongs to one tile.
 // That matters more than the padding it costs: with points numbered densely over the slab,
 // rows of different tiles shared sectors, and the stores -- not the arithmetic, nor the
 // bytes -- set the derivative stage's time.  On 16 blocks of 69^3 (4.0 M points) the stage
@@ -16,12 +17,12 @@
 // with whole sectors, and the rest of the rewrite, 0.83 and 1.14 ms.
 //
 // The algebra takes 32 points at a time along the block's rows (slab_point): two neighbouring
-// tiles' parts of a row, and, where a row has an odd number of tiles, its last part together
-// with those of the next rows.  Its accesses to the state and the right-hand side are then
-// runs of up to 32 points, and no two warps share a sector of the scratch.  (Groups of four
-// points taken densely along the rows instead left fewer lanes idle, but on 135^3 blocks,
-// whose rows of 129 points then straddle the tiles or leave a group of one point, the algebra
-// took 1.64 instead of 1.38 ms, MIXED, and 2.69 instead of 2.38 ms, FP64, on 6.4 M points.
+// tiles' parts of a row, and tiles left over together with those of the next rows (RowTasks).
+// Its accesses to the state and the right-hand side are then runs of up to 32 points, and no two
+// warps share a sector of the scratch.  (Groups of four points taken densely along the rows
+// instead left fewer lanes idle, but on 135^3 blocks, whose rows of 129 points then straddle the
+// tiles or leave a group of one point, the algebra took 1.64 instead of 1.38 ms, MIXED, and 2.69
+// instead of 2.38 ms, FP64, on 6.4 M points.
 // Two rows of one tile, whose 32 points are one block of the scratch: 1.52 and 2.46 ms.)
 #pragma once
 #include <stdint.h>
@@ -56,6 +57,18 @@ __host__ __device__ inline int cut_of(int n, int size, int pos) {
 // Scratch offset of row y of a tile within its plane: rows y and y + 2 share a 32-point
 // block, so that the derivative stage's stores, two rows apart in a warp, fill it.
 __host__ __device__ inline int row_off(int y) { return ((y & 1) << 5) | ((y & 2) << 3) | ((y & 4) << 4); }
+// Narrow tiles, of at most kNarrow columns (the last of a row can be that narrow), have rows of
+// kNarrow points, in the first half of the planes' points, the even rows before the odd ones:
+// with rows of 16, half of each 128-byte line would be unused, and memory is read by such lines.
+// (4373 blocks of 13^3, 1.5 M points, whose only tiles are 7 wide: the algebra takes 0.89 instead
+// of 1.25 ms in FP64, 0.56 instead of 0.74 ms in MIXED.  Parts of 8 and 4 columns for tiles of
+// 9 to 12 as well scattered a task's rows over more lines: 15^3 blocks took 24 % longer.)
+constexpr int kNarrow = 8;
+// Scratch offset of point (x, y) of a tile within its plane: row_off(y) + x, or the same with
+// narrow rows.
+__host__ __device__ inline int point_off(bool narrow, int x, int y) {
+  return ((y & 1) << 5) + (y >> 1 & 1) * (narrow ? kNarrow : kTileX) + (y >> 2) * (narrow ? 2 * kNarrow : 4 * kTileX) + x;
+}
 
 struct BlockDev {
   uint64_t offset;   // element offset in every variable array
@@ -72,6 +85,7 @@ struct SlabDev {
   // a strip of the planes' rows (whole tiles) where the planes are too large for the scratch:
   // first row, and how many of the block's rows it leaves out
   int32_t j0 = 0, jcut = 0;
+  int32_t narrow = 0; // its last column of tiles is narrow
 };
 // tile rows of a slab: the first one's number in the block, and how many
 __host__ __device__ inline int first_cut(const SlabDev& s) { return (s.j0 + kTileY / 2) / kTileY; }
@@ -94,47 +108,73 @@ struct SlabPoint {
   int i, j, k, lp;
   bool valid;
 };
-// How the rows of a slab of block B are cut into tasks: `tiles` parts per row, in pairs; with
-// an odd number of tiles the last parts (`lanes` lanes each) of `rows` rows share a task, which
-// follows the rows' other tasks, so that the sectors of the state and of the right-hand side
-// that it shares with them are still in L2.
+// How the rows of a slab are cut into tasks, in sets of kTaskRows rows: `pairs` pairs of tiles
+// per row; then the tiles left over, one column of them after the other -- the last, where the
+// row has an odd number of tiles or the last is narrow, and in the latter case of an even number
+// the last but one --, `lanes` lanes (0: no such column) to a row and 2^shift rows to a task.
+// They follow the set's pairs, so that the sectors of the state and of the right-hand side that
+// they share with them are still in L2.  (A narrow tile paired with the one before left up to 15
+// of 32 lanes idle: 257 blocks of 24^3, rows of 12 + 6, FP64: algebra 0.88 ms, now 0.77.)
+constexpr int kTaskRows = 8;
+struct ColumnTasks {
+  int lanes, shift;
+};
+__host__ __device__ inline ColumnTasks column(int ex) {
+  const int lanes = (ex + kGroup - 1) / kGroup * kGroup;
+  return {lanes, lanes <= 4 ? 3 : (lanes <= 8 ? 2 : 1)};
+}
 struct RowTasks {
-  int tiles, pairs, lanes, rows, tasks;  // tasks per `rows` rows
+  int tiles, pairs;
+  ColumnTasks c0, c1;  // of the last tile but one, of the last one
 };
 __host__ __device__ inline RowTasks row_tasks(int I0) {
-  const int tiles = num_cuts(I0, kTileX), pairs = tiles / 2;
-  if (tiles % 2 == 0) return {tiles, pairs, 0, 1, pairs};
-  const int lanes = (I0 - cut_start(I0, kTileX, tiles - 1) + kGroup - 1) / kGroup * kGroup, rows = 32 / lanes;
-  return {tiles, pairs, lanes, rows, rows * pairs + 1};
+  const int tiles = num_cuts(I0, kTileX), last = cut_start(I0, kTileX, tiles - 1);
+  if (tiles % 2) return {tiles, tiles / 2, {0, 0}, column(I0 - last)};
+  if (I0 - last > kNarrow) return {tiles, tiles / 2, {0, 0}, {0, 0}};
+  return {tiles, tiles / 2 - 1, column(last - cut_start(I0, kTileX, tiles - 2)), column(I0 - last)};
+}
+// tasks of `rows` rows of a left-over column, and of `rows` rows of a set
+__host__ __device__ inline int column_tasks(const ColumnTasks& c, int rows) {
+  return c.lanes ? (rows + (1 << c.shift) - 1) >> c.shift : 0;
+}
+__host__ __device__ inline int set_tasks(const RowTasks& t, int rows) {
+  return rows * t.pairs + column_tasks(t.c0, rows) + column_tasks(t.c1, rows);
 }
 // Tasks of a slab of nz planes of block B that leaves out jcut of its rows.
 __host__ __device__ inline int64_t slab_tasks(const BlockDev& B, int nz, int jcut = 0) {
   const RowTasks t = row_tasks(B.sz[0] - 6);
-  return ((int64_t)(B.sz[1] - 6 - jcut) * nz + t.rows - 1) / t.rows * t.tasks;
+  const int64_t rows = (int64_t)(B.sz[1] - 6 - jcut) * nz;
+  return rows / kTaskRows * set_tasks(t, kTaskRows) + set_tasks(t, (int)(rows % kTaskRows));
 }
 // The point of lane `lane` of a task of slab s.
 __host__ __device__ inline SlabPoint slab_point(const BlockDev& B, const SlabDev& s, int task, int lane) {
-  const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6, J = I1 - s.jcut, rows = J * s.nz;
+  const int I0 = B.sz[0] - 6, I1 = B.sz[1] - 6, J = I1 - s.jcut;
   const RowTasks t = row_tasks(I0);
-  const int set = task / t.tasks, k = task - set * t.tasks;
-  int r = set * t.rows, cx, x;  // row, its tile, point in the tile
-  if (k < t.rows * t.pairs) {
-    const int q = k / t.pairs;
-    r += q;
+  const int per_set = set_tasks(t, kTaskRows), set = task / per_set, r0 = set * kTaskRows;
+  const int rows = J * s.nz - r0 < kTaskRows ? J * s.nz - r0 : kTaskRows;  // of this set
+  int k = task - set * per_set, q, cx, x;  // row of the set, its tile, point in the tile
+  bool valid = true;
+  if (k < rows * t.pairs) {
+    q = k / t.pairs;
     cx = 2 * (k - q * t.pairs) + lane / kTileX;
     x = lane % kTileX;
   } else {
-    const int q = lane / t.lanes;
-    r = q < t.rows ? r + q : rows;
-    cx = t.tiles - 1;
-    x = lane - q * t.lanes;
+    k -= rows * t.pairs;
+    const int first = column_tasks(t.c0, rows);
+    const bool last = k >= first;
+    const ColumnTasks c = last ? t.c1 : t.c0;
+    const int p = c.lanes == 12 ? (lane >= 12 ? 1 : 0) + (lane >= 24 ? 1 : 0) : lane >> (5 - c.shift);  // lane / lanes
+    valid = p >> c.shift == 0;
+    q = ((last ? k - first : k) << c.shift) + (valid ? p : 0);
+    cx = t.tiles - (last ? 1 : 2);
+    x = lane - p * c.lanes;
   }
-  const int x0 = cut_start(I0, kTileX, cx);
-  const bool valid = r < rows && x0 + x < cut_start(I0, kTileX, cx + 1);
-  r = r < rows ? r : rows - 1;
-  const int z = r / J, y = s.j0 + r - z * J, cy = cut_of(I1, kTileY, y);
+  valid = valid && q < rows;
+  const int x0 = cut_start(I0, kTileX, cx), ex = cut_start(I0, kTileX, cx + 1) - x0;
+  const int r = r0 + (q < rows ? q : rows - 1), z = r / J, y = s.j0 + r - z * J, cy = cut_of(I1, kTileY, y);
   return {3 + x0 + x, 3 + y, 3 + s.k0 + z,
-          s.sbase + (((cy - first_cut(s)) * t.tiles + cx) * s.nz + z) * kTilePlane + row_off(y - cut_start(I1, kTileY, cy)) + x, valid};
+          s.sbase + (((cy - first_cut(s)) * t.tiles + cx) * s.nz + z) * kTilePlane +
+              point_off(s.narrow && cx == t.tiles - 1, x, y - cut_start(I1, kTileY, cy)), valid && x < ex};
 }
 
 // Which closure rows a tile's output points take: those within three points of a flagged face.

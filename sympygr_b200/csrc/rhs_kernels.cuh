@@ -340,24 +340,28 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
     __syncwarp();  // every lane is done reading the previous task's buffer
     {
       // piece lane % kPieces of the 32 points: group piece * 8 / kPieces, its first or second half
-      const int piece = lane % kPieces;
-      const int lp = __shfl_sync(0xffffffffu, p.lp, piece * (32 / kPieces) / kGroup * kGroup) + piece * (32 / kPieces) % kGroup;
+      // (FP64, bound by memory, leaves out groups without points: their first lane has none)
+      const int piece = lane % kPieces, from = piece * (32 / kPieces) / kGroup * kGroup;
+      const int lp = __shfl_sync(0xffffffffu, p.lp, from) + piece * (32 / kPieces) % kGroup;
+      const bool any = Cfg::kAll || __shfl_sync(0xffffffffu, p.valid, from);
       const uint64_t src = reinterpret_cast<uint64_t>(scr + scr_index<NS>(lane / kPieces, lp));
       constexpr int kLead = Cfg::kAll ? NS : Cfg::kFirst;  // slots from slot 0 on
 #pragma unroll 6
       for (int k = 0; k < (kLead + kPerPass - 1) / kPerPass; ++k)
-        if (kLead % kPerPass == 0 || k * kPerPass + lane / kPieces < kLead)
+        if (any && (kLead % kPerPass == 0 || k * kPerPass + lane / kPieces < kLead))
           cp_async16(dst + 512u * k, src + (uint64_t)k * (kPerPass * 32 * sizeof(ST)));
       if constexpr (!Cfg::kAll) {
 #pragma unroll 4
         for (int k = 0; k < kNumVars / kPerPass; ++k)
-          cp_async16(dst + 512u * (kLead / kPerPass + k), src + (uint64_t)(kKoSlot + k * kPerPass) * 32 * sizeof(ST));
+          if (any) cp_async16(dst + 512u * (kLead / kPerPass + k), src + (uint64_t)(kKoSlot + k * kPerPass) * 32 * sizeof(ST));
         // the slots read from global memory, into L2: one sector per group and slot
         constexpr int kGroups = kStageW / kGroup;
         const ST* const pg = scr + scr_index<NS>(0, __shfl_sync(0xffffffffu, p.lp, lane % kGroups * kGroup));
-        for (int k = Cfg::kFirst + lane / kGroups; k < kNumDerivs; k += 32 / kGroups) prefetch_l2(pg + k * 32);
-        if constexpr (ADV)
-          for (int k = kAdvSlot + lane / kGroups; k < NS; k += 32 / kGroups) prefetch_l2(pg + k * 32);
+        if (__shfl_sync(0xffffffffu, p.valid, lane % kGroups * kGroup)) {
+          for (int k = Cfg::kFirst + lane / kGroups; k < kNumDerivs; k += 32 / kGroups) prefetch_l2(pg + k * 32);
+          if constexpr (ADV)
+            for (int k = kAdvSlot + lane / kGroups; k < NS; k += 32 / kGroups) prefetch_l2(pg + k * 32);
+        }
       }
     }
     cp_async_commit();

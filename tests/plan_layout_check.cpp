@@ -94,49 +94,64 @@ static int limits() {
   return 0;
 }
 
-// Strips of planes: with a scratch too small for three planes every point still has one scratch
-// point, the one that the algebra's tasks read.
+// Every point has one scratch point, inside its buffer and no other point's, which is the one that
+// the algebra's tasks read it from, in groups of four that never straddle 32-point blocks.
+static int check_points(const std::vector<b200bssn_block>& v, const b200bssn_plan_options& o, int64_t max_scratch) {
+  const std::vector<BlockDev> dev = devices(v);
+  PlanLayout L;
+  if (lay_out(L, v.data(), dev, o, max_scratch, kSms) != B200BSSN_OK) return fail("refused", v, o);
+  std::vector<std::vector<char>> seen(v.size());
+  for (size_t b = 0; b < v.size(); ++b) seen[b].assign(Interior(v[b]).points(v[b].sz[2] - 6), 0);
+  auto id = [&](int b, int i, int j, int k) {  // interior-relative
+    return (int64_t)b << 32 | (i + Interior(v[b]).n[0] * (j + Interior(v[b]).n[1] * k));
+  };
+  for (const ChunkRec& c : L.chunks) {
+    std::vector<int64_t> owner(L.cap, -1);
+    for (int t = c.tile_begin; t < c.tile_begin + c.tile_count; ++t) {
+      const TileDev& T = L.tiles[t];
+      if (T.ex < 3 || T.ey < 3 || T.ex > kTileX || T.ey > kTileY || T.sbase % 32) return fail("tile", v, o);
+      for (int z = 0; z < T.nz; ++z)
+        for (int y = 0; y < T.ey; ++y)
+          for (int x = 0; x < T.ex; ++x) {
+            const int64_t lp = T.sbase + z * kTilePlane + point_off(T.ex <= kNarrow, x, y);
+            if (lp < 0 || lp >= L.cap) return fail("scratch point outside the buffer", v, o);
+            if (owner[lp] != -1) return fail("scratch point used twice", v, o);
+            owner[lp] = id(T.block, T.i0 + x, T.j0 + y, T.k0 + z);
+          }
+    }
+    for (int r = c.range_begin; r < c.range_begin + c.range_count; ++r)
+      for (int k = 0; k < 32 * L.ranges[r].count; ++k) {
+        const SlabDev& s = L.slabs[L.ranges[r].slab];
+        const SlabPoint p = slab_point(dev[s.block], s, L.ranges[r].start + k / 32, k % 32);
+        if (p.lp < 0 || p.lp >= L.cap) return fail("task outside the buffer", v, o);
+        if ((p.lp - k % kGroup) % kGroup) return fail("group split", v, o);
+        if (!p.valid) continue;
+        const int64_t q = id(s.block, p.i - 3, p.j - 3, p.k - 3);
+        if (owner[p.lp] != q) return fail("the algebra reads another point", v, o);
+        if (seen[s.block][(int32_t)q]++) return fail("point taken twice", v, o);
+      }
+  }
+  for (const auto& w : seen)
+    for (const char s : w)
+      if (!s) return fail("point left out", v, o);
+  return 0;
+}
+
+static int points() {
+  b200bssn_plan_options o{};
+  for (uint32_t n = 13; n <= 151; ++n) {  // every width of the last tiles, whole and ragged rows
+    o.slab_depth = n % 7;
+    if (check_points({block_of(n, 13 + n * 5 % 29, 13 + n * 3 % 17), block_of(13 + n % 19, n, 14)}, o, max_scratch_points(162))) return 1;
+  }
+  return 0;
+}
+
+// planes of which no three fit the scratch
 static int strips() {
   for (const int I1 : {7, 9, 17, 18, 31, 64, 65, 66})
-    for (const int64_t rows : {1, 2, 3}) {
-      const int I0 = 40, I2 = 13;
-      const std::vector<b200bssn_block> v{block_of(I0 + 6, I1 + 6, I2 + 6), block_of(19, 23, 17)};
-      const b200bssn_plan_options o{};
-      const std::vector<BlockDev> dev = devices(v);
-      PlanLayout L;
-      if (lay_out(L, v.data(), dev, o, rows * 3 * 4 * kTilePlane, kSms) != B200BSSN_OK) return fail("refused", v, o);
-      std::vector<std::vector<char>> seen(2);
-      for (int b = 0; b < 2; ++b) seen[b].assign(Interior(v[b]).points(v[b].sz[2] - 6), 0);
-      for (const ChunkRec& c : L.chunks) {
-        std::vector<int64_t> owner(L.cap, -1);
-        auto id = [&](int b, int i, int j, int k) {  // interior-relative
-          return (int64_t)b << 32 | (i + Interior(v[b]).n[0] * (j + Interior(v[b]).n[1] * k));
-        };
-        for (int t = c.tile_begin; t < c.tile_begin + c.tile_count; ++t) {
-          const TileDev& T = L.tiles[t];
-          for (int z = 0; z < T.nz; ++z)
-            for (int y = 0; y < T.ey; ++y)
-              for (int x = 0; x < T.ex; ++x) {
-                int64_t& w = owner[T.sbase + z * kTilePlane + row_off(y) + x];
-                if (w != -1) return fail("scratch point used twice", v, o);
-                w = id(T.block, T.i0 + x, T.j0 + y, T.k0 + z);
-              }
-        }
-        for (int r = c.range_begin; r < c.range_begin + c.range_count; ++r)
-          for (int k = 0; k < 32 * L.ranges[r].count; ++k) {
-            const SlabDev& s = L.slabs[L.ranges[r].slab];
-            const SlabPoint p = slab_point(dev[s.block], s, L.ranges[r].start + k / 32, k % 32);
-            if (p.lp < 0 || p.lp >= L.cap) return fail("scratch point outside the buffer", v, o);
-            if (!p.valid) continue;
-            const int64_t q = id(s.block, p.i - 3, p.j - 3, p.k - 3);
-            if (owner[p.lp] != q) return fail("the algebra reads another point", v, o);
-            if (seen[s.block][(int32_t)q]++) return fail("point taken twice", v, o);
-          }
-      }
-      for (const auto& w : seen)
-        for (const char s : w)
-          if (!s) return fail("point left out", v, o);
-    }
+    for (const int64_t rows : {1, 2, 3})
+      for (const int I0 : {40, 44, 48})
+        if (check_points({block_of(I0 + 6, I1 + 6, 19), block_of(19, 23, 17)}, {}, rows * 3 * 4 * kTilePlane)) return 1;
   return 0;
 }
 
@@ -144,6 +159,7 @@ int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   int rc = 2;
   if (what == "limits") rc = limits();
+  if (what == "points") rc = points();
   if (what == "strips") rc = strips();
   if (rc == 0) std::puts("ok");
   return rc;
