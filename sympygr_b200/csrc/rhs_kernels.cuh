@@ -314,9 +314,14 @@ bssn_algebra_staged_kernel(const __grid_constant__ AlgebraArgs a, int ntasks) {
   const uint32_t dst = static_cast<uint32_t>(__cvta_generic_to_shared(sd)) + 16u * (uint32_t)lane;
   const int nwarps = gridDim.x * Cfg::kWarps;
   // Neighbouring tasks share state and scratch lines and go to one CTA; fewer tasks than warps
-  // are spread over the SMs first.
-  const int first = ntasks < nwarps ? warp * gridDim.x + blockIdx.x : blockIdx.x * Cfg::kWarps + warp;
-  for (int task = first; task < ntasks; task += nwarps) {
+  // are spread over the SMs first.  From one round of tasks to the next every warp's place moves
+  // on by one: tasks with face points take longer and recur with the rows, and at the same place
+  // half of the warps could meet nearly all of them (135^3, MIXED, all faces flagged, where
+  // they recur every 34 tasks: a call took 4 % longer).
+  int place = ntasks < nwarps ? warp * gridDim.x + blockIdx.x : blockIdx.x * Cfg::kWarps + warp;
+  for (int round = 0; round < ntasks; round += nwarps, place = place + 1 < nwarps ? place + 1 : 0) {
+    const int task = round + place;
+    if (task >= ntasks) continue;
     const RangeDev rg = a.ranges[a.range_base + task / kRangeTasks];
     if ((task & (kRangeTasks - 1)) >= rg.count) continue;
     const SlabDev slab = a.slabs[rg.slab];
