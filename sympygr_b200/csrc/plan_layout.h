@@ -142,9 +142,12 @@ inline int lay_out(PlanLayout& L, const b200bssn_block* blocks, const std::vecto
     const int cutx = num_cuts(I0, kTileX), c0 = first_cut(u), cuty = cut_rows(I1, u);
     const int64_t points = (int64_t)I0 * (I1 - u.jcut) * u.nz, need = (int64_t)cutx * cuty * u.nz * kTilePlane;
     // a block's slabs stay in one chunk when the whole block fits in one
-    const int64_t block_pts = (int64_t)I0 * I1 * (B.sz[2] - 6);
+    const Interior in(blocks[u.block]);
+    const int64_t block_pts = in.points(in.n[2]), block_need = in.plane * in.n[2];
     const bool first = si == 0 || L.slabs[si - 1].block != u.block;
-    if (first && block_pts <= capacity && cur.points + block_pts > capacity) flush();
+    if (first && block_pts <= capacity && block_need <= max_scratch &&
+        (cur.points + block_pts > capacity || used + block_need > max_scratch))
+      flush();
     if (cur.points + points > capacity || used + need > max_scratch) flush();
     cur.points += points;
     u.sbase = (int32_t)used;

@@ -155,12 +155,50 @@ static int strips() {
   return 0;
 }
 
+// Blocks that fit a chunk are not split between chunks (the host-array path overlaps its copies
+// only then).
+static int check_whole(const std::vector<b200bssn_block>& v, const b200bssn_plan_options& o) {
+  PlanLayout L;
+  const int64_t max_scratch = max_scratch_points(num_slots(o.advective != 0));
+  if (lay_out(L, v.data(), devices(v), o, max_scratch, kSms) != B200BSSN_OK) return fail("refused", v, o);
+  std::vector<int> chunk(v.size(), -1);
+  for (size_t c = 0; c < L.chunks.size(); ++c)
+    for (int t = L.chunks[c].tile_begin; t < L.chunks[c].tile_begin + L.chunks[c].tile_count; ++t) {
+      const int b = L.tiles[t].block;
+      const Interior in(v[b]);
+      const int64_t capacity = o.chunk_points ? (int64_t)o.chunk_points : int64_t(1) << 23;
+      if (chunk[b] >= 0 && chunk[b] != (int)c && in.points(in.n[2]) <= capacity && in.plane * in.n[2] <= max_scratch)
+        return fail("block split between chunks", v, o);
+      chunk[b] = (int)c;
+    }
+  return 0;
+}
+
+static int whole() {
+  for (int adv = 0; adv < 2; ++adv) {
+    b200bssn_plan_options o{};
+    o.advective = adv;
+    for (const int count : {4, 23})
+      for (const uint32_t n : {135u, 151u, 167u, 175u, 200u})
+        if (check_whole(std::vector<b200bssn_block>(count, block_of(n, n, n)), o)) return 1;
+    std::vector<b200bssn_block> mixed;
+    for (int k = 0; k < 3000; ++k) mixed.push_back(block_of(13 + k % 3, 13 + k % 5, 13));
+    for (int k = 0; k < 12; ++k) mixed.push_back(block_of(135 + 9 * (k % 4), 140, 130));
+    for (const uint64_t points : {0, 2200000, 3000000, 5000000}) {
+      o.chunk_points = points;
+      if (check_whole(mixed, o)) return 1;
+    }
+  }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   int rc = 2;
   if (what == "limits") rc = limits();
   if (what == "points") rc = points();
   if (what == "strips") rc = strips();
+  if (what == "whole") rc = whole();
   if (rc == 0) std::puts("ok");
   return rc;
 }
