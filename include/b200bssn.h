@@ -109,16 +109,21 @@ int b200bssn_rhs(b200bssn_ctx *ctx, double *const *rhs, const double *const *u,
 
 /* Work plan for a fixed block list: descriptors, tiles and the derivative
  * scratch live on the device.  Build once, evaluate many times (RK stages).
- * `chunk_points` bounds the interior points evaluated per kernel pair (and so the
- * scratch: 1296 bytes per point in FP64, 648 in MIXED, and what pads rows to tiles of 16 x 8
- * points: 4 % for 63^3 points, 18 % for 129^3); 0 picks the default. */
+ * `chunk_points` (0 picks the default, 2^23) bounds the points evaluated per group of
+ * launches, and so the scratch, of 1296 bytes per scratch point in FP64 and 648 in MIXED
+ * (upwind mode 1873 and 937): as many scratch points for a plan whose interior points fit
+ * one chunk, twice as many (two buffers) for others, and never fewer than one of its
+ * slabs, or of its blocks of no more interior points than that, needs; up to 2^20 per
+ * buffer only the interior points count towards it.  A block's scratch
+ * points are its interior points with rows and columns padded to tiles of 16 x 8: 4 % more
+ * for 63^3 points and 18 % for 129^3, but 161 % for 7^3, and 216 % for planes of 9 x 9. */
 int b200bssn_plan_create(b200bssn_ctx *ctx, const b200bssn_block *blocks, uint32_t nblocks,
                          uint32_t precision, uint64_t chunk_points, b200bssn_plan **plan);
 int b200bssn_plan_destroy(b200bssn_plan *plan);
 
 /* Tuning knobs of a plan (0 in any field: the default). */
 typedef struct b200bssn_plan_options {
-  uint64_t chunk_points;       /* interior points per kernel pair (scratch size) */
+  uint64_t chunk_points;       /* points per group of launches, and of the scratch (see above) */
   uint32_t slab_depth;         /* max interior z planes per work unit, but never fewer than 3; fewer
                                 * where that many do not fit the largest scratch (default: by a cost
                                 * model of the whole plan).  A plan is refused with

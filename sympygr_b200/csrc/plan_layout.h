@@ -11,7 +11,7 @@
 
 namespace b200bssn {
 
-constexpr int64_t kDefaultChunkPoints = int64_t(1) << 23;
+constexpr int64_t kDefaultChunkPoints = int64_t(1) << 23, kSmallScratch = int64_t(1) << 20;
 // A plan is refused when a z-slab of the depth asked for (kNominalDepth planes where none is)
 // holds more interior points than max_chunk_points.  The slabs that are made may be thinner.
 constexpr int64_t kNominalDepth = 48;
@@ -66,16 +66,17 @@ inline int64_t default_depth(const b200bssn_block* blocks, size_t nblocks, int64
   int64_t best = 3;
   double best_cost = 0.0;
   for (const int64_t depth : {3, 4, 5, 6, 8, 11, 16, 22, 33, 44, 66, 99, 132}) {
-    double work = 0.0, points = 0.0;
+    double work = 0.0, points = 0.0, scratch = 0.0;
     int64_t longest = 0;
     for (size_t b = 0; b < nblocks; ++b) {
       const Interior in(blocks[b]);
       const int64_t n = in.slabs(depth, limit);
       work += (double)(in.cutx * in.cuty) * (double)(in.n[2] + 10 * n);
       points += (double)in.points(in.n[2]);
+      scratch += (double)(in.plane * in.n[2]);
       longest = std::max(longest, (in.n[2] + n - 1) / n + 10);
     }
-    const double launches = std::max(1.0, points / (double)capacity);
+    const double launches = std::max({1.0, points / (double)capacity, scratch / (double)limit});
     const double cost = work * kLongerKindVars / resident + launches * (double)longest;
     if (best_cost == 0.0 || cost < best_cost) {
       best_cost = cost;
@@ -103,14 +104,34 @@ inline int lay_out(PlanLayout& L, const b200bssn_block* blocks, const std::vecto
     max_slab = std::max(max_slab, points);
   }
   if (max_slab > kMaxChunkPoints) return B200BSSN_ERR_SIZE_LIMIT;
-  // interior points of a chunk
+  // Interior points of a chunk, and the scratch points of a buffer.  Padding takes part of the
+  // latter: a plan of several chunks has two buffers of at most `capacity` scratch points each,
+  // and a plan whose interior points fit one chunk no more than that in all -- in two buffers
+  // where its scratch points do not fit one --, but for whole blocks and slabs of the depth asked
+  // for, which are not cut for this, and for kSmallScratch points, which padding may always take:
+  // smaller chunks cost more time than the memory is worth (305 blocks of 23^3, MIXED, chunks
+  // of 60,000 points: 2.69 ms when these include the padding, 2.08 ms when they do not).
   const int64_t capacity = std::min(std::max(o.chunk_points ? (int64_t)o.chunk_points : kDefaultChunkPoints, max_slab), kMaxChunkPoints);
-
-  // The slabs; in planes of which no three fit the scratch, strips of a slab's tile rows.
-  const int64_t model_depth = default_depth(blocks, nblocks, capacity, max_scratch, sms);
+  int64_t limit = std::min(capacity, max_scratch), all_points = 0, all_need = 0, whole = 0;
   for (size_t b = 0; b < nblocks; ++b) {
     const Interior in(blocks[b]);
-    const int64_t n = in.slabs(depth_asked(b) ? depth_asked(b) : model_depth, max_scratch);
+    const int64_t points = in.points(in.n[2]), need = in.plane * in.n[2];
+    all_points += points;
+    all_need += need;
+    if (points <= capacity && need <= max_scratch) whole = std::max(whole, need);
+    const int64_t depth = depth_asked(b) ? depth_asked(b) : kNominalDepth, n = (in.n[2] + depth - 1) / depth;
+    const int64_t slab = in.plane * ((in.n[2] + n - 1) / n);
+    if (slab <= max_scratch) whole = std::max(whole, slab);
+  }
+  if (all_points <= capacity && all_need > limit) limit /= 2;
+  limit = std::max({limit, whole, std::min(kSmallScratch, max_scratch)});
+  if (all_points <= capacity && all_need <= std::min(2 * limit, max_scratch)) limit = std::max(limit, all_need);
+
+  // The slabs; in planes of which no three fit the scratch, strips of a slab's tile rows.
+  const int64_t model_depth = default_depth(blocks, nblocks, capacity, limit, sms);
+  for (size_t b = 0; b < nblocks; ++b) {
+    const Interior in(blocks[b]);
+    const int64_t n = in.slabs(depth_asked(b) ? depth_asked(b) : model_depth, limit);
     for (int64_t sl = 0; sl < n; ++sl) {
       const int64_t k0 = sl * in.n[2] / n, nz = (sl + 1) * in.n[2] / n - k0;
       int per = in.cuty;  // rows of tiles per strip
@@ -119,6 +140,7 @@ inline int lay_out(PlanLayout& L, const b200bssn_block* blocks, const std::vecto
       for (int c = 0; c < in.cuty; c += per) {
         const int j0 = cut_start(I1, kTileY, c), j1 = cut_start(I1, kTileY, std::min(c + per, in.cuty));
         L.slabs.push_back({(int32_t)b, (int32_t)k0, (int32_t)nz, 0, j0, I1 - (j1 - j0), in.narrow()});
+        limit = std::max(limit, (int64_t)in.cutx * std::min(per, in.cuty - c) * kTilePlane * nz);
       }
     }
   }
@@ -145,10 +167,10 @@ inline int lay_out(PlanLayout& L, const b200bssn_block* blocks, const std::vecto
     const Interior in(blocks[u.block]);
     const int64_t block_pts = in.points(in.n[2]), block_need = in.plane * in.n[2];
     const bool first = si == 0 || L.slabs[si - 1].block != u.block;
-    if (first && block_pts <= capacity && block_need <= max_scratch &&
-        (cur.points + block_pts > capacity || used + block_need > max_scratch))
+    if (first && block_pts <= capacity && block_need <= limit &&
+        (cur.points + block_pts > capacity || used + block_need > limit))
       flush();
-    if (cur.points + points > capacity || used + need > max_scratch) flush();
+    if (cur.points + points > capacity || used + need > limit) flush();
     cur.points += points;
     u.sbase = (int32_t)used;
     for (int ty = 0; ty < cuty; ++ty)

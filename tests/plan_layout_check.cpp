@@ -192,6 +192,28 @@ static int whole() {
   return 0;
 }
 
+// The scratch of lists of small blocks, whose padding weighs most: as many scratch points as
+// chunk_points for a plan whose interior points fit one chunk, twice as many for others.
+static int memory() {
+  for (int adv = 0; adv < 2; ++adv)
+    for (const uint32_t n : {13u, 14u, 15u, 17u, 21u, 23u, 37u})
+      for (const int64_t points : {30000, 2000000, 6860000, 12000000})
+        for (const int64_t chunk : {0, 20000, 300000, 3000000}) {
+          b200bssn_plan_options o{};
+          o.advective = adv;
+          o.chunk_points = chunk;
+          const Interior in(block_of(n, n, n));
+          const std::vector<b200bssn_block> v(points / in.points(in.n[2]) + 1, block_of(n, n, n));
+          PlanLayout L;
+          if (lay_out(L, v.data(), devices(v), o, max_scratch_points(num_slots(adv != 0)), kSms) != B200BSSN_OK) return fail("refused", v, o);
+          const int64_t capacity = chunk ? chunk : int64_t(1) << 23, all = in.points(in.n[2]) * (int64_t)v.size();
+          int64_t bound = all <= capacity ? capacity : 2 * capacity;
+          bound = std::max(bound, int64_t(2) << 20);  // small scratch buffers may be padded beyond it
+          if (L.cap * (L.chunks.size() > 1 ? 2 : 1) > bound) return fail("scratch larger than asked for", v, o);
+        }
+  return 0;
+}
+
 int main(int argc, char** argv) {
   const std::string what = argc > 1 ? argv[1] : "";
   int rc = 2;
@@ -199,6 +221,7 @@ int main(int argc, char** argv) {
   if (what == "points") rc = points();
   if (what == "strips") rc = strips();
   if (what == "whole") rc = whole();
+  if (what == "memory") rc = memory();
   if (rc == 0) std::puts("ok");
   return rc;
 }

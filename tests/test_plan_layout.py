@@ -18,8 +18,9 @@ def checker(tmp_path_factory):
 
 # limits: no plan is refused whose slabs of the depth asked for (48 planes by default) fit, none is
 # accepted whose slabs do not; points: tiles and algebra tasks agree on every point's scratch point;
-# strips: the same with planes larger than the scratch; whole: blocks that fit a chunk are not split
-@pytest.mark.parametrize("check", ["limits", "points", "strips", "whole"])
+# strips: the same with planes larger than the scratch; whole: blocks that fit a chunk are not split;
+# memory: scratch buffers hold no more points than asked for, the tiles' padding among them
+@pytest.mark.parametrize("check", ["limits", "points", "strips", "whole", "memory"])
 def test_plan_layout(checker, check):
     res = subprocess.run([checker, check], capture_output=True, text=True)
     assert res.returncode == 0 and res.stdout.strip() == "ok", res.stdout
