@@ -26,6 +26,13 @@ namespace b200bssn {
 
 constexpr int kNumConstraints = 4;  // ham, mom0, mom1, mom2
 
+// What the constraint algebra reads, as ranges [first, end): variables, and derivative slots
+// (the first derivatives of these variables, the second ones of gt and chi).
+struct ReadRanges {
+  int first0, end0, first1, end1;
+};
+constexpr ReadRanges kConstraintVars{1, 6, 12, 24}, kConstraintSlots{3, 18, 36, 114};
+
 struct ConstraintArgs {
   const double* u[kNumVars];
   double* con[kNumConstraints];  // all null: fields not written
@@ -72,19 +79,27 @@ bssn_constraints_kernel(const __grid_constant__ ConstraintArgs a) {
   const bool active = task < rg.count && p.valid;
   if (sizeof(ST) == 8) {
     // FP64 (latency bound at 255 registers): pull the run's scratch into L2 first, so
-    // the per-point loads below hit L2: one sector per group and derivative slot that the
-    // constraints read.  (MIXED, closer to the DRAM bound, lost 3 % to the extra
+    // the per-point loads below hit L2: one sector per group with points and derivative slot
+    // that the constraints read.  (MIXED, closer to the DRAM bound, lost 3 % to the extra
     // instructions.)
-    const ST* const own = static_cast<const ST*>(a.scr) + scr_index(a.nslots, 0, p.lp - (int)(threadIdx.x % kGroup));
-    for (int s = threadIdx.x % kGroup; s < kNumDerivs; s += kGroup) prefetch_l2(own + s * 32);
+    const int in_group = threadIdx.x % kGroup;
+    const ST* const own = static_cast<const ST*>(a.scr) + scr_index(a.nslots, 0, p.lp - in_group);
+    if (__shfl_sync(0xffffffffu, active, threadIdx.x % 32 - in_group)) {
+      constexpr ReadRanges r = kConstraintSlots;
+      for (int s = r.first0 + in_group; s < r.end0; s += kGroup) prefetch_l2(own + s * 32);
+      for (int s = r.first1 + in_group; s < r.end1; s += kGroup) prefetch_l2(own + s * 32);
+    }
   }
   double sq[kNumConstraints] = {0.0, 0.0, 0.0, 0.0};
   double mx[kNumConstraints] = {0.0, 0.0, 0.0, 0.0};
   if (active) {
     const int64_t pp = B.offset + p.i + (int64_t)B.sz[0] * (p.j + (int64_t)B.sz[1] * p.k);
     if (sizeof(ST) == 8) {
+      constexpr ReadRanges r = kConstraintVars;
 #pragma unroll
-      for (int v = 0; v < kNumVars; ++v) prefetch_l2(a.u[v] + pp);
+      for (int v = r.first0; v < r.end0; ++v) prefetch_l2(a.u[v] + pp);
+#pragma unroll
+      for (int v = r.first1; v < r.end1; ++v) prefetch_l2(a.u[v] + pp);
     }
     ConstraintIn<RT, ST> in{&a, pp, p.lp};
     ConstraintSink<RT> sink;
