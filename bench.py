@@ -44,7 +44,7 @@ MIXED_BAR = 1e-6
 #  * the stencils: 105 first derivatives (72 + 33 mixed) x 12, 33 diagonal second
 #    derivatives x 14, 72 KO rows x 14, the KO add 24 x 4, eta damping ~10.
 # FP64 path: all of it in FP64.  MIXED: the algebra in FP32, the stencils in FP64
-# (their differences; the weighted sums of the split-precision rows run in FP32).
+# (rounded to FP32 when they are stored).
 FLOPS_ALGEBRA = 4137
 FLOPS_STENCIL = 105 * 12 + 33 * 14 + 72 * 14 + 24 * 4 + 10
 # Bytes per interior point an evaluation must move at the least: the 24 state
@@ -350,10 +350,12 @@ def reference_arm(args, rank, world):
 
 
 def roofline(kernel, ms, npts, bytes_pp, f64_pp, f32_pp, hbm_peak, peak64, peak32, traffic_pp=None,
-             launches=1, peak_src=""):
+             launches=None, peak_src=""):
     """Roofline of one kernel (or a whole evaluation) from algorithmic work per point:
     `achieved`/`peak` against HBM (the contract's object), the FP64/FP32 pipe time
-    beside it, and which roof binds (the longer of the two lower bounds)."""
+    beside it, and which roof binds (the longer of the two lower bounds).  `traffic`: DRAM
+    bytes of a step, all launches together; `launches`: how many there are, None where only
+    the evaluation's are counted."""
     secs = ms * 1e-3
     gbs = bytes_pp * npts / secs / 1e9
     t_hbm = bytes_pp * npts / (hbm_peak * 1e9)
@@ -361,7 +363,7 @@ def roofline(kernel, ms, npts, bytes_pp, f64_pp, f32_pp, hbm_peak, peak64, peak3
     t_pipe = max(f64_pp * npts / (peak64 * 1e12), f32_pp * npts / (peak32 * 1e12))
     out = {"kernel": kernel, "bound": "hbm", "achieved": round(gbs, 1), "peak": hbm_peak, "unit": "GB/s",
            "frac": round(gbs / hbm_peak, 4),
-           "traffic": None if traffic_pp is None else round(traffic_pp * npts / launches),
+           "traffic": None if traffic_pp is None else round(traffic_pp * npts), "traffic_scope": "step",
            "bytes_per_point": round(bytes_pp, 1), "launches_per_step": launches,
            "peak_source": peak_src,
            "pipe": {"fp64_flops_per_point": f64_pp, "fp32_flops_per_point": f32_pp,
@@ -777,15 +779,16 @@ def main():
             # not algorithmic (the reference's algorithm needs no scratch traffic)
             "derivs": roofline(f"bssn_derivs_kind_kernel<{'float' if mode == 'mixed' else 'double'},*> (all launches)",
                                d_ms, npts, read_state, FLOPS_STENCIL, 0, hbm_peak, peak64, peak32,
-                               tr["derivs"], 1, peak_src),
+                               tr["derivs"], None, peak_src),
             # algebra: the state at the point in, the 24 right-hand sides out
             "algebra": roofline(f"bssn_algebra_staged_kernel<{'float' if mode == 'mixed' else 'double'},0>",
                                 a_ms, npts, 2 * BYTES_VARS, f64_alg, f32_alg, hbm_peak, peak64, peak32,
-                                tr["algebra"], 1, peak_src),
+                                tr["algebra"], None, peak_src),
             "evaluation": roofline(f"whole {mode} evaluation (all launches)",
                                    ms_mixed if mode == "mixed" else ms_fp64, npts,
                                    read_state + BYTES_VARS, FLOPS_STENCIL + f64_alg, f32_alg,
-                                   hbm_peak, peak64, peak32, tr["derivs"] + tr["algebra"], 1, peak_src),
+                                   hbm_peak, peak64, peak32, tr["derivs"] + tr["algebra"],
+                                   plans[prec].launches, peak_src),
         }
 
     # the single-block configurations and the end-to-end legs run after the batch's
