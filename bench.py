@@ -55,8 +55,8 @@ BYTES_VARS = 24 * 8
 # large blocks (four 69^3 and one 135^3, one flagged face): `python bench.py
 # --profile-case {mixed,fp64} [--single-pass]` (derivative stage: its kernels summed;
 # the one-pass kernel with its default 128-slot ring).
-NCU_TRAFFIC_PER_POINT = {"mixed": {"derivs": 895.0, "algebra": 1409.0, "single_pass": 836.0},
-                         "fp64": {"derivs": 1573.0, "algebra": 1943.0}}
+NCU_TRAFFIC_PER_POINT = {"mixed": {"derivs": 894.0, "algebra": 1100.0, "single_pass": 712.0},
+                         "fp64": {"derivs": 1570.0, "algebra": 1861.0}}
 REF_STEP_CAP, REF_WARMUP_CAP = 3, 1  # reference arm: ~32 s per full-batch step on 16 threads
 
 PG_TIMEOUT_S = 120  # process-group timeout under torchrun (N > 1)

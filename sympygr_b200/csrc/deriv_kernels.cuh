@@ -17,13 +17,13 @@
 //     D_z(D_y).  unroll_planes planes are processed per loop pass, so the register windows
 //     move once per pass.
 //
-// What bounds it: see plan_types.h for the stores.  The kernel that this one replaced (one
-// column per thread, CTAs of 4 warps, 8-byte copies, one plane per barrier and pass) kept the
-// shared-memory data pipe 81 / 70 % busy (without / with second derivatives) once its stores
-// filled whole sectors; sharing the y windows, 16-byte copies and the unrolled passes bring that
-// to 59 %, the issue slots to 65 / 60 % and DRAM to 52 / 44 % of its peak (64 blocks of 37^3,
-// MIXED): no single resource is full, and what is left is the latency of 16 / 12 warps per SM.
-// 16 blocks of 69^3 (4.0 M points): 0.83 ms (MIXED) and 1.14 ms (FP64), before 1.46 and 2.00 ms.
+// What bounds it: see plan_types.h for the stores.  With one column per thread, CTAs of 4
+// warps, 8-byte copies and one plane per barrier and pass, the shared-memory data pipe is 81 /
+// 70 % busy (without / with second derivatives) once the stores fill whole sectors; sharing the
+// y windows, 16-byte copies and the unrolled passes bring that to 59 %, the issue slots to 65 /
+// 60 % and DRAM to 52 / 44 % of its peak (64 blocks of 37^3, MIXED): no single resource is full,
+// and what is left is the latency of 16 / 12 warps per SM.  16 blocks of 69^3 (4.0 M points):
+// 0.83 ms (MIXED) and 1.14 ms (FP64), in that other form 1.46 and 2.00 ms.
 //
 // Closure rows (within three points of a flagged face) reach no further than three points
 // beyond a tile or slab (cut_start).  Along z the three rows of a face are formed together,
@@ -37,7 +37,7 @@
 // of every warp, they took tiles at such faces 3.5 times as long as others.  64 blocks of 37^3
 // with all faces flagged: 0.93 ms (MIXED) and 1.03 ms (FP64); with the z rows copied out and
 // every thread working out its closure points anew in each plane 1.10 and 1.25 ms; 0.46 and
-// 0.60 ms without faces.  16 blocks of 69^3: 1.39 and 1.62 ms, before 3.65 and 4.13 ms.
+// 0.60 ms without faces.  16 blocks of 69^3: 1.39 and 1.62 ms.
 #pragma once
 #include <cuda_runtime.h>
 #include <stdint.h>
@@ -690,9 +690,9 @@ __device__ __forceinline__ void derive_item(const DerivArgs& a, const BlockDev& 
 }
 
 // Upwind mode: the signs of the shift at every scratch point of a chunk's tiles, one CTA of
-// kTilePlane threads per tile.  (Each derivative item used to read the shift itself: three
-// loads of 8 bytes per point, direction and variable, waited for at once; a byte per point
-// and variable, a plane ahead, replaces them.)  Columns that pad a tile take its last one's.
+// kTilePlane threads per tile.  (A derivative item that reads the shift itself has
+// three loads of 8 bytes per point, direction and variable, waited for at once; this way it has
+// a byte per point, a plane ahead.)  Columns that pad a tile take its last one's.
 static __global__ void __launch_bounds__(kTilePlane)
 bssn_shift_signs_kernel(const double* b0, const double* b1, const double* b2, const BlockDev* blocks, const TileDev* tiles,
                         uint8_t* up) {
@@ -729,8 +729,7 @@ constexpr int kKindVars[2] = {13, 11};        // [DD]
 // it start at once, so its CTAs fill the SMs as the ones before run out of items, and the
 // launches of a small plan run side by side.  A CTA ends only when the launch before has
 // ended, so that the last launch's end is the stage's.  (A call on one 21^3 block with all
-// faces flagged, MIXED, whose launches last 20-30 us each, takes 80 us; 166 us before the
-// kernels, the slabs and this.)
+// faces flagged, MIXED, whose launches last 20-30 us each, takes 80 us.)
 constexpr int kind_ctas_per_sm(bool dd, bool adv, int closure) {
   return dd ? (adv ? 4 : 6) : (closure == kClosureXY ? 6 : 8);
 }

@@ -278,9 +278,9 @@ __device__ __forceinline__ void algebra_point_at(const AlgebraArgs& a, const Blo
   } else if constexpr (sizeof(RT) == 8) {
     // FP64: the algebra in two parts (the six At_rhs with the Ricci tensor, then the
     // rest), each with its own live set: the opaque offset between them keeps the compiler from
-    // holding values of the first for the second.  At 255 registers what spills -- 72 bytes --
-    // counts: shared memory leaves little L1, and the same kernel with 340 bytes took 1.60
-    // instead of 1.36 ms on 16 blocks of 69^3
+    // holding values of the first for the second.  At 255 registers what spills -- 40 bytes --
+    // counts: shared memory leaves little L1, and the same kernel with 72 and 340 bytes took
+    // 1.36 and 1.60 instead of 1.32 ms on 16 blocks of 69^3
     RhsAlgebraPart<0>::run<RT>(in, sink, *prm, (RT)eta);
     asm volatile("" : "+l"(in.pp));
     RhsAlgebraPart<1>::run<RT>(in, sink, *prm, (RT)eta);
