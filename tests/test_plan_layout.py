@@ -9,7 +9,7 @@ REPO = os.path.dirname(HERE)
 
 
 @pytest.fixture(scope="module")
-def checker(tmp_path_factory):
+def layout_check(tmp_path_factory):
     exe = str(tmp_path_factory.mktemp("layout") / "plan_layout_check")
     subprocess.run(["g++", "-O2", "-std=c++17", "-Wall", "-I", os.path.join(REPO, "sympygr_b200", "csrc"), "-I", os.path.join(REPO, "include"),
                     os.path.join(HERE, "plan_layout_check.cpp"), "-o", exe], check=True)
@@ -21,6 +21,6 @@ def checker(tmp_path_factory):
 # strips: the same with planes larger than the scratch; whole: blocks that fit a chunk are not split;
 # memory: scratch buffers hold no more points than asked for, the tiles' padding among them
 @pytest.mark.parametrize("check", ["limits", "points", "strips", "whole", "memory"])
-def test_plan_layout(checker, check):
-    res = subprocess.run([checker, check], capture_output=True, text=True)
+def test_plan_layout(layout_check, check):
+    res = subprocess.run([layout_check, check], capture_output=True, text=True)
     assert res.returncode == 0 and res.stdout.strip() == "ok", res.stdout
